@@ -70,9 +70,13 @@ def latent_attention(h, w, mx, eps, positions=None):
     return out.reshape(T, H * V) @ w["o"].T
 
 
-def mlstm(h, w, mx, eps, state=None):
+def mlstm(h, w, mx, eps, state=None, first=None, flip=()):
     """Matrix-memory recurrence, token by token.  Returns (output [T, E], state) where state is
-    (S [H, dim, vdim], n [H, dim], m [H]); a sequence starts with zeros, m included."""
+    (S [H, dim, vdim], n [H, dim], m [H]); a sequence starts with zeros, m included.
+
+    The first token's read-out is a multiple of (k . q) v, which the norm divides by its own size: v with the sign of
+    k . q.  `first`: a list that gets |k . q| / (|k| |q|) per head of that token.  `flip`: heads for which that one
+    read-out takes the other sign."""
     T = h.shape[0]
     H, D, V, cap = mx["heads"], mx["dim"], mx["vdim"], mx["gate_cap"]
     q = (h @ w["q"].T).reshape(T, H, D) * D ** -0.5
@@ -94,6 +98,10 @@ def mlstm(h, w, mx, eps, state=None):
             n[a] = keep * n[a] + add * k[t, a]
             m[a] = m_new
             o[t, a] = S[a].T @ q[t, a] / (max(abs(n[a] @ q[t, a]), math.exp(-m_new)) + 1e-6)
+    if first is not None:
+        first.append(np.abs((q[0] * k[0]).sum(-1)) / (np.linalg.norm(q[0], axis=-1) * np.linalg.norm(k[0], axis=-1)))
+    for a in flip:
+        o[0, a] = -o[0, a]
     o = rms_unit(o, eps).reshape(T, H * V) * w["norm"]
     gate = 1.0 / (1.0 + np.exp(-(h @ w["g"].T)))
     return (o * gate) @ w["o"].T, (S, n, m)
@@ -153,9 +161,10 @@ def sub(weights, prefix):
     return {k[len(prefix):]: np.asarray(v, dtype=np.float64) for k, v in weights.items() if k.startswith(prefix)}
 
 
-def forward(config, weights, tokens, return_layers=False, margins=None):
+def forward(config, weights, tokens, return_layers=False, margins=None, first=None, flips=()):
     """Logits [T, vocab] of one whole sequence (and the residual stream after every layer).  `margins`: a list
-    that gets, for every layer with routed experts, each token's distance from another choice (see `route`)."""
+    that gets, for every layer with routed experts, each token's distance from another choice (see `route`).
+    `first`, `flips`: for every matrix memory what `mlstm` reports, as (layer, ratios); (layer, head) pairs to flip."""
     eps = config["norm"]["eps"]
     x = np.asarray(weights["embed"], dtype=np.float64)[np.asarray(tokens)]
     after = []
@@ -165,7 +174,10 @@ def forward(config, weights, tokens, return_layers=False, margins=None):
         if layer["type"] == "latent_attention":
             y = latent_attention(h, mw, layer["mixer"], eps)
         elif layer["type"] == "mlstm":
-            y, _ = mlstm(h, mw, layer["mixer"], eps)
+            ratios = []
+            y, _ = mlstm(h, mw, layer["mixer"], eps, first=ratios, flip=[a for j, a in flips if j == i])
+            if first is not None:
+                first.append((i, ratios[0]))
         else:
             raise ValueError(layer["type"])
         mlp = layer.get("mlp")

@@ -57,26 +57,52 @@ def model_of(seed):
 
 
 @functools.lru_cache(maxsize=None)
-def plain_of(seed, tokens):
+def plain_of(seed, tokens, flips=frozenset()):
+    """(logits, every token's distance from another choice of experts, the undecided (layer, head) pairs)."""
     cfg, w = model_of(seed)
-    margins = []
-    logits = plain.forward(cfg, w, list(tokens), margins=margins)
-    return logits, (np.min(np.stack(margins), axis=0) if margins else np.full(len(tokens), np.inf))
+    margins, first = [], []
+    logits = plain.forward(cfg, w, list(tokens), margins=margins, first=first, flips=flips)
+    margin = np.min(np.stack(margins), axis=0) if margins else np.full(len(tokens), np.inf)
+    return logits, margin, [(i, a) for i, ratios in first for a, r in enumerate(ratios) if r <= UNDECIDED]
+
+
+# The read-out of a sequence's first token in a matrix memory is v times the SIGN of k . q, whatever its size.  A bfloat16
+# run knows k . q to about |k| |q| 2^-8 only: the rows that k and q are products of are rounded to 8 bits of mantissa, and
+# each part before them adds an error of 0.002 to 0.004 of its output (2^-8 = 0.0039).  Below that either sign is right.
+UNDECIDED = 2.0 ** -8
+
+
+def plain_runs(seed, tokens):
+    """The plain run first, then those that differ from it in the sign of undecided first read-outs."""
+    todo, seen = [frozenset()], set()
+    while todo:
+        flips = todo.pop(0)
+        if flips in seen:
+            continue
+        seen.add(flips)
+        logits, margin, undecided = plain_of(seed, tokens, flips)
+        assert len(undecided) <= 2, "a configuration that a bfloat16 run cannot be held to"
+        todo += [flips | {pair} for pair in undecided]
+        yield logits, margin
 
 
 def compare(got, seed, tokens, dtype, what):
-    want, margin = plain_of(seed, tuple(tokens))
+    """float32 runs: against the plain run.  bfloat16 runs: against the plain run with one choice of the signs that
+    bfloat16 leaves undecided, the same choice for all positions (the one that the run is closest to)."""
     got = np.asarray(got)
+    runs = list(plain_runs(seed, tuple(tokens)))
     if dtype == "bfloat16":
         # a router's choice closer than 0.08 logits may fall the other way in bfloat16 and changes the positions
         # after it too: the run is compared up to the first such position
-        close_calls = np.nonzero(margin <= 0.08)[0]
-        upto = int(close_calls[0]) if len(close_calls) else len(margin)
         assert np.isfinite(got).all(), what
-        if upto:
-            check_logits(got[:upto], want[:upto], dtype, what)
+        close_calls = [np.nonzero(margin <= 0.08)[0] for _, margin in runs]
+        uptos = [int(c[0]) if len(c) else len(got) for c in close_calls]
+        best = min((i for i in range(len(runs)) if uptos[i] >= uptos[0]),      # (none that compares fewer positions)
+                   key=lambda i: np.abs(got[:uptos[i]] - runs[i][0][:uptos[i]]).max(initial=0.0))
+        if uptos[best]:
+            check_logits(got[:uptos[best]], runs[best][0][:uptos[best]], dtype, what)
         return
-    diff = np.abs(got.astype(np.float64) - want)
+    diff = np.abs(got.astype(np.float64) - runs[0][0])
     assert np.isfinite(got).all() and diff.max() <= 2e-4 and diff.mean() <= 1e-5, \
         f"{what}: max |diff| {diff.max():.3e}, mean {diff.mean():.3e}"
 
