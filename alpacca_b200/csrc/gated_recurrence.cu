@@ -16,8 +16,8 @@
 // column's dot products run in four chains per lane; the lanes' shares of a read-out wait in shared memory and are
 // added after the round, so that the walk of a decay per channel has no exchange between lanes and no barrier in
 // it (the delta rule needs one exchange per token, S^T k over all rows, by shuffles).  The order of additions depends
-// on the column alone, so a token's output is bitwise the same in any step that this walk serves.
-// Prompts of mode 0 (`ab_gla_prompt`) walk pieces of a sequence side by side instead (piece_walk.cuh): the same 32-bit
+// on the column alone, so a token's output is bitwise the same in a prompt, a portion or a step of one token.
+// Prompts of mode 0 in a bfloat16 model (`ab_gla_prompt`) walk pieces of a sequence side by side instead (piece_walk.cuh): the same 32-bit
 // operations, the state before a piece added up from its predecessors'.
 //
 // Around it: the decays of mode 0 (sigmoid(z)^(1/tau) with z = W_2 y + b from the low-rank projection's first half y) come

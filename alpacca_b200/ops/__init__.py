@@ -1066,13 +1066,14 @@ def mlstm_state_row(D: int, V: int) -> int:
 
 
 def mlstm_step(proj, offsets, bias_i, bias_f, state, ctx, H, D, V, cap, qscale, norm_weight, eps, out,
-               write_state=True):
+               write_state=True, in_order=False):
     """The matrix-memory recurrence over the step's tokens, from each sequence's state to its new state.
 
     proj float32 [T, N]: one row per token with q | k | v | g | zi | zf at `offsets` (six column offsets);
     state float32 [slots, H, mlstm_state_row(D, V)]; out [T, H*V] of the activation dtype gets
     o / rms(o per head) * norm_weight * sigmoid(g).  Sequences, slots and padding rows are taken from the
-    context's device arrays (cu_q, slots, tok_seq)."""
+    context's device arrays (cu_q, slots, tok_seq).  `in_order`: every state is walked token by token, so that a sequence's
+    numbers do not depend on what else is in the step (prompts in pieces depend on it in their last bits)."""
     _cuda(proj, bias_i, bias_f, state, norm_weight, out)
     T, B = ctx.n_tokens, ctx.n_seqs
     off_q, off_k, off_v, off_g, off_i, off_f = (int(o) for o in offsets)
@@ -1094,7 +1095,7 @@ def mlstm_step(proj, offsets, bias_i, bias_f, state, ctx, H, D, V, cap, qscale, 
     _i32(ctx.tok_seq, T, "tok_seq")
     coef = torch.empty((T, H, 3), dtype=torch.float32, device=proj.device)
     o_raw = torch.empty((T, H, V + 1), dtype=torch.float32, device=proj.device)
-    if _walks_pieces(ctx, D, V) and not (off_q | off_k | off_v | ld) % 4 and not (proj.data_ptr() | state.data_ptr()) % 16:
+    if not in_order and _walks_pieces(ctx, D, V) and not (off_q | off_k | off_v | ld) % 4 and not (proj.data_ptr() | state.data_ptr()) % 16:
         length, pieces, local, prod = _piece_scratch(ctx, H, D, V + 4, 1, proj.device)
         _check(_lib("mlstm").ab_mlstm_prompt(
             _p(proj), ld, off_q, off_k, off_v, off_g, off_i, off_f, _p(bias_i), _p(bias_f), _p(state), row, H, D, V,
@@ -1991,12 +1992,14 @@ def _f32_rows(t, n, name):
 
 
 def gated_recurrence(mode, q, k, v, state, out, ctx, H, Hk, D, V, qscale=1.0, decay=None, beta=None, skip=None,
-                     write_state=True):
+                     write_state=True, in_order=False):
     """One walk of a recurrent mixer over the step's tokens; q, k [T, Hk * D] and v [T, H * V] float32 (views with a
     row stride are fine), state float32 [slots, H, D, V], out float32 [T, H * V].
     mode "channel": S <- diag(a_t) S + k_t v_t^T, o_t = S^T (q_t qscale), decay a [T, H * D];
     mode "delta": S <- g_t S; u = beta_t (v_t - S^T k_t); S <- S + k_t u^T; o_t = S^T (q_t qscale), decay g and beta [T, H];
-    mode "scalar": S <- g_t S + beta_t k_t v_t^T, o_t = S^T q_t + skip_h v_t, decay g and beta [T, H], skip [H] or None."""
+    mode "scalar": S <- g_t S + beta_t k_t v_t^T, o_t = S^T q_t + skip_h v_t, decay g and beta [T, H], skip [H] or None.
+    `in_order`: token by token, whatever the step's lengths: a token's numbers are then the same bits alone, in any batch and
+    under any cut into steps (mode "channel" walks prompts in pieces otherwise, the other modes never do)."""
     _cuda(q, k, v, state, out, decay, beta, skip)
     T = ctx.n_tokens
     _need(mode in ("channel", "delta", "scalar"), "gated_recurrence: mode channel, delta or scalar")
@@ -2022,7 +2025,7 @@ def gated_recurrence(mode, q, k, v, state, out, ctx, H, Hk, D, V, qscale=1.0, de
         ldd, dvec, dsc = 0, None, decay
     _i32(ctx.cu_q, ctx.n_seqs + 1, "cu_q")
     _i32(ctx.slots, ctx.n_seqs, "slots")
-    if (mode == "channel" and H == Hk and _walks_pieces(ctx, D, V) and not (ldq | ldk | ldv | ldd) % 4
+    if (mode == "channel" and H == Hk and not in_order and _walks_pieces(ctx, D, V) and not (ldq | ldk | ldv | ldd) % 4
             and not (q.data_ptr() | k.data_ptr() | v.data_ptr() | decay.data_ptr() | state.data_ptr()) % 16):
         length, pieces, local, prod = _piece_scratch(ctx, H, D, V, D, q.device)
         _check(_lib("gated_recurrence").ab_gla_prompt(

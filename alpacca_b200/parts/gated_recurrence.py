@@ -79,7 +79,7 @@ class GatedLinearAttention(Mixer):
         o = torch.empty((proj.shape[0], H * V), dtype=torch.float32, device=proj.device)
         ops.gated_recurrence("channel", proj[:, oq:oq + H * D], proj[:, ok:ok + H * D], proj[:, ov:ov + H * V],
                              cache.state, o, ctx, H, H, D, V, qscale=float(D) ** -0.5, decay=decay,
-                             write_state=write_cache)
+                             write_state=write_cache, in_order=self.opts.dtype == torch.float32)
         mixed = torch.empty((proj.shape[0], H * V), dtype=self.opts.dtype, device=proj.device)
         ops.head_norm_gate(o, self.norm_weight, proj[:, og:og + H * V], "silu", self.eps, mixed, ctx, H, V)
         return self.out.forward(mixed, n_rows=T)

@@ -65,5 +65,6 @@ class MatrixMemory(Mixer):
         proj = self.proj.forward(h, n_rows=T)
         mixed = torch.empty((proj.shape[0], self.H * self.V), dtype=self.opts.dtype, device=proj.device)
         ops.mlstm_step(proj, self.offsets, self.bias_i, self.bias_f, cache.state, ctx, self.H, self.D, self.V, self.cap,
-                       self.D ** -0.5, self.norm_weight, self.eps, mixed, write_state=write_cache)
+                       self.D ** -0.5, self.norm_weight, self.eps, mixed, write_state=write_cache,
+                       in_order=self.opts.dtype == torch.float32)
         return self.out.forward(mixed, n_rows=T)

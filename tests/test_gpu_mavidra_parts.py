@@ -503,3 +503,39 @@ def test_walk_in_pieces(D, V):
                 assert ((out[t].view(H, V).double() - o).abs() <= (2 * (t - at + 1) + D + 4) * 2.0 ** -24 * bound).all(), (slot, t - at)
             assert ((state[slot].double() - S).abs() <= (2 * n + 4) * 2.0 ** -24 * B).all() if write else torch.equal(state[slot], before[slot])
             at += n
+
+
+@pytest.mark.parametrize("mixer", ["gated linear attention", "matrix memory"])
+def test_float32_prompt_does_not_depend_on_the_step(mixer):
+    """A 32-bit model's recurrence is walked in the order of the tokens: a prompt's rows and state are the same bits alone and
+    beside neighbours of other lengths, those of the gated linear attention under any cut into steps too."""
+    from alpacca_b200.parts import GatedLinearAttention, MatrixMemory
+    width, H, D, V = 40, 2, 64, 128
+    opts = opts_of("float32")
+    if mixer == "matrix memory":
+        part = MatrixMemory(opts, width, H, D, V, 12.0, 1e-5, "m")
+    else:
+        part = GatedLinearAttention(opts, width, H, D, V, 16, 16.0, 1e-5, "m", out_dtype=torch.float32)
+    load_part(part, seed=3)
+    x = torch.randn((300, width), generator=torch.Generator("cuda").manual_seed(1), device="cuda")
+    others = torch.randn((900, width), generator=torch.Generator("cuda").manual_seed(2), device="cuda")
+
+    def run(before, cuts, after):
+        hs = PartHarness([part.cache_spec()], "float32", max_tokens=8192, max_positions=4096)
+        slots = [hs.cache.alloc_slot() for _ in range(3)]
+        rows, at = [], 0
+        for n in cuts:
+            seqs = [(s, n_) for s, n_ in zip(slots, (before, n, after)) if n_]
+            ctx = hs.step(seqs)
+            h = torch.cat([others[:before], x[at:at + n], others[:after]]).contiguous()
+            view = hs.cache.entry_view(0, ctx.block_tables)
+            rows.append(part.forward(h, ctx, view)[before:before + n].float())
+            hs.done()
+            at += n
+        return torch.cat(rows), view.state[slots[1]].clone()
+    want, state = run(0, (300,), 0)
+    cuts = [(300,)] if mixer == "matrix memory" else [(300,), (100, 200), (1, 299), (64, 1, 235)]
+    for cut in cuts:
+        for before, after in ((0, 0), (0, 900), (70, 0), (1, 450)):
+            rows, s = run(before, cut, after)
+            assert torch.equal(rows, want) and torch.equal(s, state), (cut, before, after)
