@@ -1299,8 +1299,8 @@ def moe_route(h, router, n_tokens, groups, keep, top, scale, bias=None, score="s
     `score` "sigmoid" (or "logit"): the scores are sigmoid(z) (or z); the choice is made by score + `correction`
     (float32 [E], if given), a group's score is the sum of its `group_top` largest choice scores, and the weights are
     the chosen experts' scores without the correction, divided by their sum only if `renorm`.
-    `router16`: the router's matrix in bfloat16, where that holds it exactly: bfloat16 rows then run a library product with a
-    float32 result (many tokens; the products are exact, the sums 32-bit), or read half the bytes (few)."""
+    `router16`: the router's matrix in bfloat16, where that holds it exactly: few bfloat16 rows then read half the bytes; many,
+    with scores that are no softmax, run a library product with a float32 result (the products are exact)."""
     _cuda(h, router, bias, correction, router16)
     _need(router16 is None or (router16.dtype == torch.bfloat16 and router16.shape == router.shape and router16.is_contiguous()),
           "moe_route: router16 bfloat16 [experts, width]")
@@ -1342,12 +1342,6 @@ def moe_route(h, router, n_tokens, groups, keep, top, scale, bias=None, score="s
             _p(h), _dt(h), width, _p(router), _p(bias), _p(correction), n_tokens, width, E, groups, keep, int(group_top),
             top, MOE_SCORES[score], 1 if renorm else 0, ctypes.c_float(scale), _p(z), _p(idx), _p(wts), _stream()),
             "moe_route", kernels=2)
-        return idx, wts
-    if w16 is not None and bias is None and n_tokens > MOE_ROUTE_SMALL_MAX_ROWS:
-        z = torch.mm(h.view(-1, width)[:n_tokens], w16.t(), out_dtype=torch.float32)
-        _mark("library product")
-        _check(_lib("moe").ab_moe_route_softmax(_p(z), n_tokens, E, groups, keep, top, ctypes.c_float(scale), _p(idx), _p(wts),
-                                                _stream()), "moe_route")
         return idx, wts
     _check(_lib("moe").ab_moe_route_bias(_p(h), _dt(h), width, _p(router), _p(bias), n_tokens, width, E, groups, keep,
                                          top, ctypes.c_float(scale), _p(z), _p(idx), _p(wts), _stream()),
