@@ -343,19 +343,19 @@ AB_API int ab_gated_recurrence(int mode, const float* q, int ldq, const float* k
   return ab_launch_status();
 }
 
-// Mode 0 for a step that brings many tokens per sequence.  `length` tokens per piece, `pieces` of the longest sequence; with more than one, local [n_seqs, H, pieces,
-// D, V] and prod [n_seqs, H, pieces, D] floats of scratch.
+// Mode 0 for a step that brings many tokens per sequence.  `length` tokens per piece; `items` pieces of all sequences, `kept` of
+// those that have more than one; local [kept, H, D, V] and prod [kept, H, D] floats of scratch.
 AB_API int ab_gla_prompt(const float* q, int ldq, const float* k, int ldk, const float* v, int ldv, const float* decay, int ldd,
                          float qscale, float* state, float* out, const int* cu_q, const int* slots, int n_seqs, int H, int D,
-                         int V, int write_state, int pieces, int length, float* local, float* prod, cudaStream_t stream) {
+                         int V, int write_state, int length, int items, int kept, float* local, float* prod, cudaStream_t stream) {
   if (n_seqs <= 0) return AB_OK;
-  if (H <= 0 || !piece_walk_takes(D, V) || (pieces > 1 && (!local || !prod))) return AB_BAD_ARG;
+  if (H <= 0 || !piece_walk_takes(D, V)) return AB_BAD_ARG;
   if ((ldq | ldk | ldv | ldd) % 4 ||
       (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)decay | (uintptr_t)state | (uintptr_t)local) & 15))
     return AB_BAD_ARG;
-  const PieceArgs w{q, k, v, ldq, ldk, ldv, decay, ldd, nullptr, state, D * V, out, V, cu_q, slots, H, V, pieces, length, 0, qscale,
-                    write_state, local, prod};
-  return piece_walk<true, false>(w, D, n_seqs, stream);
+  const PieceArgs w{q, k, v, ldq, ldk, ldv, decay, ldd, nullptr, state, D * V, out, V, cu_q, slots, n_seqs, H, V, length, items, kept, 0,
+                    qscale, write_state, local, prod};
+  return piece_walk<true, false>(w, D, stream);
 }
 
 // Per token: the convolution over the token's and the `taps - 1` inputs before it, per channel, of the first `Cc` =

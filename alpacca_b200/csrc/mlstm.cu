@@ -447,26 +447,26 @@ static int launch_output(const float* o_raw, const float* proj, int ld, int off_
   return ab_launch_status();
 }
 
-// A step that brings many tokens per sequence.  `length` tokens per piece, `pieces` of the longest sequence; with more than one, local [n_seqs, H, pieces, D, V + 4]
-// and prod [n_seqs, H, pieces] floats of scratch.
+// A step that brings many tokens per sequence.  `length` tokens per piece; `items` pieces of all sequences, `kept` of those that
+// have more than one; local [kept, H, D, V + 4] and prod [kept, H] floats of scratch.
 AB_API int ab_mlstm_prompt(const float* proj, int ld, int off_q, int off_k, int off_v, int off_g, int off_i, int off_f,
                            const float* bias_i, const float* bias_f, float* state, int row, int H, int D, int V,
                            const int* cu_q, const int* slots, const int* tok_seq, int n_seqs, int n_tokens, float cap,
                            float qscale, float* coef, float* o_raw, const float* weight, float eps, void* out,
-                           int out_dtype, int write_state, int pieces, int length, float* local, float* prod,
+                           int out_dtype, int write_state, int length, int items, int kept, float* local, float* prod,
                            cudaStream_t stream) {
   if (n_seqs <= 0 || n_tokens <= 0) return AB_OK;
-  if (H <= 0 || n_seqs > 65535 || row < D * V + D + 1 || row % 4 || !piece_walk_takes(D, V) || (pieces > 1 && (!local || !prod)))
+  if (H <= 0 || n_seqs > 65535 || row < D * V + D + 1 || row % 4 || !piece_walk_takes(D, V))
     return AB_BAD_ARG;
-  if ((off_q | off_k | off_v | ld) % 4 || (((uintptr_t)proj | (uintptr_t)state) & 15)) return AB_BAD_ARG;
+  if ((off_q | off_k | off_v | ld) % 4 || (((uintptr_t)proj | (uintptr_t)state | (uintptr_t)local) & 15)) return AB_BAD_ARG;
   MlstmArgs a{proj, ld, off_q, off_k, off_v, off_g, off_i, off_f, bias_i, bias_f, state, row, H, D, V, cu_q, slots,
               tok_seq, cap, qscale, coef, o_raw, write_state};
   ab_launch(mlstm_scan_runs_kernel, dim3((unsigned)H, (unsigned)n_seqs), dim3(32 * SCAN_WARPS), 0, stream, a);
   int rc = ab_launch_status();
   if (rc) return rc;
   const PieceArgs w{proj + off_q, proj + off_k, proj + off_v, ld, ld, ld, nullptr, 0, coef, state, row, o_raw, V + 1, cu_q,
-                    slots, H, V, pieces, length, 0, qscale, write_state, local, prod};
-  rc = piece_walk<false, true>(w, D, n_seqs, stream);
+                    slots, n_seqs, H, V, length, items, kept, 0, qscale, write_state, local, prod};
+  rc = piece_walk<false, true>(w, D, stream);
   if (rc) return rc;
   return launch_output(o_raw, proj, ld, off_g, weight, tok_seq, out, out_dtype, n_tokens, H, V, eps, coef, 1, stream);
 }

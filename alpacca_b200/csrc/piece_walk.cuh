@@ -16,9 +16,11 @@
 // operations per number of S and token with a decay per row, and half as much again for the local pass.
 // One sequence of 2,048 tokens, 8 heads of 128 x 256 with one decay each, the whole mixer 522 -> 258 us (the walk token by
 // token with one column per thread 448 us); 2,500 tokens of two sequences, 16 heads of 128 x 128 with a decay per row, the
-// whole mixer with its decays out of the 32-bit product (150 -> 40 us) 898 -> 331 us (the walk 640).
-// Pieces of one length for all sequences, no more than run at once, and lanes that never leave the exchanges: 274 -> 258, 371 ->
-// 331 us against pieces counted per sequence.
+// whole mixer with its decays out of the 32-bit product 898 -> 331 us (the walk 640).
+// Pieces of one length for all sequences, as many as run at once (or in two rounds), and lanes that never leave the exchanges: 274
+// -> 258, 371 -> 331 us against pieces counted per sequence.  A long prompt beside rows of one token is cut like a prompt alone:
+// matrix memory, 8 heads, 2,048 + 17 x 1 tokens 1,300 -> 278 us, 8,192 + 11 x 1 3,073 -> 976, against a room shared by number of
+// sequences; eight of 2,000 to 3,750 tokens in two rounds 3,109 -> 2,569.
 #pragma once
 #include "common.cuh"
 #include "launch.cuh"
@@ -38,12 +40,13 @@ struct PieceArgs {
   float* out;                  // out + (t * H + h) * out_row + column
   int out_row;
   const int *cu_q, *slots;
-  int H, V, pieces, length;    // pieces of the longest sequence, tokens per piece
+  int n_seqs, H, V, length;    // tokens per piece
+  int items, kept;             // pieces of all sequences, and of those that have more than one (the host's sums)
   int cols;                    // columns per CTA, a multiple of 4 (set by the launch)
   float qscale;
   int write_state;
-  float* local;                // pieces > 1: [n_seqs, H, pieces][D][V + (WITH_N ? 4 : 0)]
-  float* prod;                 // [n_seqs, H, pieces][CHANNEL ? D : 1]
+  float* local;                // [kept, H][D][V + (WITH_N ? 4 : 0)]
+  float* prod;                 // [kept, H][CHANNEL ? D : 1]
 };
 
 typedef unsigned long long f32x2;
@@ -70,14 +73,48 @@ __device__ __forceinline__ void pw_copy4(float* dst, const float* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
 }
 
-// a piece's tokens: `len` of them, a multiple of PW_TOKENS, but for a sequence's last piece
+// A piece: `length` of its sequence's tokens (a multiple of PW_TOKENS), the last one what is left.  Items count the pieces of
+// all sequences one after another; every warp finds its own by itself, 32 sequences at a time, from the lengths on the device.
 struct Piece {
+  int b = -1;          // sequence; -1: no such item
+  int n = 0, p = 0;    // its pieces, and which of them
+  int at = 0;          // the sequence's first place in `local` (n > 1)
   int begin, end;
-  bool last;
-  __device__ __forceinline__ Piece(int t0, int t1, int len, int p) {
-    begin = min(t1, t0 + p * len);
-    end = min(t1, begin + len);
-    last = end == t1;          // (an empty piece too: the caller looks at begin < end)
+  // by_sequence: `item` is a sequence (begin and end are all of its tokens)
+  __device__ __forceinline__ Piece(const int* __restrict__ cu_q, int n_seqs, int length, int item, bool by_sequence) {
+    const int lane = threadIdx.x & 31;
+    int items = 0, kept = 0;
+    for (int base = 0; base < n_seqs; base += 32) {
+      const int i = base + lane;
+      const int t0 = cu_q[min(i, n_seqs)], t1 = cu_q[min(i + 1, n_seqs)];
+      const unsigned pieces = (unsigned)(t1 - t0 + length - 1) / (unsigned)length;
+      const unsigned word = pieces | (pieces > 1 ? pieces << 16 : 0u);      // both sums in one: 65,535 items at most
+      unsigned up = word;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned v = __shfl_up_sync(0xffffffffu, up, o);
+        if (lane >= o) up += v;
+      }
+      const unsigned hit = __ballot_sync(0xffffffffu, by_sequence ? i == item : items + (int)(up & 0xffffu) > item);
+      if (hit) {
+        const int l = __ffs(hit) - 1;
+        const unsigned before = __shfl_sync(0xffffffffu, up - word, l);
+        b = base + l;
+        n = (int)__shfl_sync(0xffffffffu, pieces, l);
+        at = kept + (int)(before >> 16);
+        begin = __shfl_sync(0xffffffffu, t0, l);
+        end = __shfl_sync(0xffffffffu, t1, l);
+        if (!by_sequence) {
+          p = item - items - (int)(before & 0xffffu);
+          begin += p * length;
+          end = min(end, begin + length);
+        }
+        return;
+      }
+      const unsigned all = __shfl_sync(0xffffffffu, up, 31);
+      items += (int)(all & 0xffffu);
+      kept += (int)(all >> 16);
+    }
   }
 };
 
@@ -158,7 +195,7 @@ __device__ __forceinline__ void stage_round(float* base, const PieceArgs& a, int
 __device__ __forceinline__ void pw_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void pw_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(PW_STAGES - 2) : "memory"); }
 
-// grid (tiles of columns, H, n_seqs * (pieces - 1))
+// grid (tiles of columns, H, items)
 template <int J, bool CHANNEL, bool WITH_N>
 __global__ void __launch_bounds__(8 * PW_COLS / 4, J <= 4 ? 2 : 1) piece_local_kernel(PieceArgs a) {
   using R = PieceRound<J, CHANNEL, false>;
@@ -166,9 +203,11 @@ __global__ void __launch_bounds__(8 * PW_COLS / 4, J <= 4 ? 2 : 1) piece_local_k
   extern __shared__ __align__(16) float pw_sm[];
   pdl_wait();
   pdl_trigger();
-  const int b = blockIdx.z / (a.pieces - 1), p = blockIdx.z % (a.pieces - 1), h = blockIdx.y;
-  const Piece piece(a.cu_q[b], a.cu_q[b + 1], a.length, p);
-  if (a.slots[b] < 0 || piece.begin >= piece.end || piece.last) return;      // nothing follows the last piece
+  const int h = blockIdx.y;
+  const Piece piece(a.cu_q, a.n_seqs, a.length, blockIdx.z, false);
+  if (piece.b < 0 || piece.p + 1 >= piece.n || a.slots[piece.b] < 0) return;      // nothing follows the last piece
+  __shared__ int kept_place;                     // SCALAR: needed after the walk, whose registers are all taken
+  if (!CHANNEL && threadIdx.x == 0) kept_place = piece.at + piece.p;
   const PieceLane me(a.V + (WITH_N ? 4 : 0), a.cols);
   const bool is_n = WITH_N && me.c0 >= a.V;
   const int rounds = (piece.end - piece.begin) / PW_TOKENS;                  // whole ones: the piece is not the last
@@ -224,7 +263,7 @@ __global__ void __launch_bounds__(8 * PW_COLS / 4, J <= 4 ? 2 : 1) piece_local_k
   }
   if (!me.live) return;
   const int VW = a.V + (WITH_N ? 4 : 0);
-  const size_t at = ((size_t)b * a.H + h) * a.pieces + p;
+  const size_t at = (size_t)(CHANNEL ? piece.at + piece.p : kept_place) * a.H + h;      // (written before the first round's barrier)
   tile_store<J>(m, a.local + at * D * VW + me.c0, VW, me.dg);
   if (blockIdx.x == 0 && me.c0 == 0) {
     if (CHANNEL) {
@@ -246,29 +285,31 @@ template <bool CHANNEL, bool WITH_N>
 __global__ void __launch_bounds__(256) piece_scan_kernel(PieceArgs a, int D) {
   pdl_wait();
   pdl_trigger();
-  const int b = blockIdx.z, h = blockIdx.y, VW = a.V + (WITH_N ? 4 : 0);
+  const int h = blockIdx.y, VW = a.V + (WITH_N ? 4 : 0);
   const int i = blockIdx.x * 256 + threadIdx.x;
-  const int slot = a.slots[b], t0 = a.cu_q[b], t1 = a.cu_q[b + 1];
-  if (slot < 0 || t1 <= t0 || i >= D * (VW / 4)) return;
+  const Piece seq(a.cu_q, a.n_seqs, a.length, blockIdx.z, true);
+  if (seq.n < 2) return;                         // walked from the sequence's state as it stands
+  const int slot = a.slots[seq.b], n = seq.n;
+  if (slot < 0 || i >= D * (VW / 4)) return;
   const int d = i / (VW / 4), c = i % (VW / 4) * 4;
   const float* st = a.state + ((size_t)slot * a.H + h) * a.state_row;
   float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
   if (c < a.V) s = *reinterpret_cast<const float4*>(st + (size_t)d * a.V + c);
   else s.x = st[(size_t)D * a.V + d];            // n
-  const size_t first = ((size_t)b * a.H + h) * a.pieces;
+  const size_t first = (size_t)seq.at * a.H + h;
   float* l = a.local + first * D * VW + (size_t)d * VW + c;
   const float* f = a.prod + first * (CHANNEL ? D : 1) + (CHANNEL ? d : 0);
-  const size_t step = (size_t)D * VW;
-  const int n = (t1 - t0 + a.length - 1) / a.length;      // the sequence's pieces
+  const size_t step = (size_t)a.H * D * VW, f_step = (size_t)a.H * (CHANNEL ? D : 1);
   float4 next = make_float4(0.f, 0.f, 0.f, 0.f);
   float keep = 0.f;
-  if (n > 1) { next = *reinterpret_cast<const float4*>(l); keep = f[0]; }
+  next = *reinterpret_cast<const float4*>(l);
+  keep = f[0];
   for (int p = 0; p < n; ++p) {
     const float4 own = next;
     const float g = keep;
     if (p + 2 < n) {                             // asked for before the store that might hold it up
       next = *reinterpret_cast<const float4*>(l + (p + 1) * step);
-      keep = f[(size_t)(p + 1) * (CHANNEL ? D : 1)];
+      keep = f[(p + 1) * f_step];
     }
     *reinterpret_cast<float4*>(l + p * step) = s;
     s.x = fmaf(g, s.x, own.x);
@@ -278,7 +319,7 @@ __global__ void __launch_bounds__(256) piece_scan_kernel(PieceArgs a, int D) {
   }
 }
 
-// grid (tiles of columns, H, n_seqs * pieces)
+// grid (tiles of columns, H, items)
 template <int J, bool CHANNEL, bool WITH_N>
 __global__ void __launch_bounds__(8 * PW_COLS / 4, J <= 4 ? 2 : 1) piece_walk_kernel(PieceArgs a) {
   using R = PieceRound<J, CHANNEL, true>;
@@ -286,10 +327,12 @@ __global__ void __launch_bounds__(8 * PW_COLS / 4, J <= 4 ? 2 : 1) piece_walk_ke
   extern __shared__ __align__(16) float pw_sm[];
   pdl_wait();
   pdl_trigger();
-  const int b = blockIdx.z / a.pieces, p = blockIdx.z % a.pieces, h = blockIdx.y;
-  const Piece piece(a.cu_q[b], a.cu_q[b + 1], a.length, p);
-  const int slot = a.slots[b];
-  if (slot < 0 || piece.begin >= piece.end) return;
+  const int h = blockIdx.y;
+  const Piece piece(a.cu_q, a.n_seqs, a.length, blockIdx.z, false);
+  const int slot = piece.b < 0 ? -1 : a.slots[piece.b];
+  if (slot < 0) return;
+  __shared__ int last_of;                        // SCALAR: needed after the walk, whose registers are all taken
+  if (!CHANNEL && threadIdx.x == 0) last_of = piece.p + 1 < piece.n ? -1 : slot;
   const PieceLane me(a.V + (WITH_N ? 4 : 0), a.cols);
   const bool is_n = WITH_N && me.c0 >= a.V;
   auto stage = [&](int r) {
@@ -302,8 +345,8 @@ __global__ void __launch_bounds__(8 * PW_COLS / 4, J <= 4 ? 2 : 1) piece_walk_ke
   float* st = a.state + ((size_t)slot * a.H + h) * a.state_row;
   if (me.live) {
     const int VW = a.V + (WITH_N ? 4 : 0);
-    if (a.pieces > 1) {
-      tile_load<J>(m, a.local + (((size_t)b * a.H + h) * a.pieces + p) * D * VW + me.c0, VW, me.dg);
+    if (piece.n > 1) {
+      tile_load<J>(m, a.local + ((size_t)(piece.at + piece.p) * a.H + h) * D * VW + me.c0, VW, me.dg);
     } else if (!is_n) {
       tile_load<J>(m, st + me.c0, a.V, me.dg);
     } else {
@@ -372,7 +415,8 @@ __global__ void __launch_bounds__(8 * PW_COLS / 4, J <= 4 ? 2 : 1) piece_walk_ke
       }
     }
   }
-  if (!a.write_state || !piece.last || !me.live) return;
+  if (!a.write_state || !me.live || (CHANNEL ? piece.p + 1 < piece.n : last_of < 0)) return;
+  if (!CHANNEL) st = a.state + ((size_t)last_of * a.H + h) * a.state_row;
   if (!is_n) {
     tile_store<J>(m, st + me.c0, a.V, me.dg);
   } else {
@@ -392,7 +436,7 @@ static inline bool piece_walk_takes(int D, int V) {
 }
 
 template <int J, bool CHANNEL, bool WITH_N>
-static int piece_walk_go(PieceArgs a, int n_seqs, cudaStream_t stream) {
+static int piece_walk_go(PieceArgs a, cudaStream_t stream) {
   const int D = 32 * J, width = a.V + (WITH_N ? 4 : 0), tiles = (width + PW_COLS - 1) / PW_COLS;
   a.cols = ((width + tiles - 1) / tiles + 3) / 4 * 4;
   const dim3 block((a.cols + 15) / 16 * 32);
@@ -401,28 +445,30 @@ static int piece_walk_go(PieceArgs a, int n_seqs, cudaStream_t stream) {
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(piece_walk_kernel<J, CHANNEL, WITH_N>, cudaFuncAttributeMaxDynamicSharedMemorySize, walk_smem);
   if (e != cudaSuccess) return AB_CUDA_ERR + (int)e;
-  if (a.pieces > 1) {
-    ab_launch(piece_local_kernel<J, CHANNEL, WITH_N>, dim3(tiles, a.H, n_seqs * (a.pieces - 1)), block, local_smem, stream, a);
+  if (a.kept > 0) {
+    ab_launch(piece_local_kernel<J, CHANNEL, WITH_N>, dim3(tiles, a.H, a.items), block, local_smem, stream, a);
     int rc = ab_launch_status();
     if (rc) return rc;
     const int quads = D * (width / 4);
-    ab_launch(piece_scan_kernel<CHANNEL, WITH_N>, dim3((quads + 255) / 256, a.H, n_seqs), dim3(256), 0, stream, a, D);
+    ab_launch(piece_scan_kernel<CHANNEL, WITH_N>, dim3((quads + 255) / 256, a.H, a.n_seqs), dim3(256), 0, stream, a, D);
     rc = ab_launch_status();
     if (rc) return rc;
   }
-  ab_launch(piece_walk_kernel<J, CHANNEL, WITH_N>, dim3(tiles, a.H, n_seqs * a.pieces), block, walk_smem, stream, a);
+  ab_launch(piece_walk_kernel<J, CHANNEL, WITH_N>, dim3(tiles, a.H, a.items), block, walk_smem, stream, a);
   return ab_launch_status();
 }
 
 template <bool CHANNEL, bool WITH_N>
-static int piece_walk(const PieceArgs& a, int D, int n_seqs, cudaStream_t stream) {
-  if (!piece_walk_takes(D, a.V) || a.pieces < 1 || a.length < 1 || a.length % PW_TOKENS || a.H > 65535 || (long long)n_seqs * a.pieces > 65535) return AB_BAD_ARG;
+static int piece_walk(const PieceArgs& a, int D, cudaStream_t stream) {
+  if (!piece_walk_takes(D, a.V) || a.length < 1 || a.length % PW_TOKENS || a.H > 65535 || a.n_seqs > 65535 || a.items < 1 ||
+      a.items > 65535 || a.kept < 0 || (a.kept > 0 && (!a.local || !a.prod)))
+    return AB_BAD_ARG;
   switch (D / 32) {
-    case 1: return piece_walk_go<1, CHANNEL, WITH_N>(a, n_seqs, stream);
-    case 2: return piece_walk_go<2, CHANNEL, WITH_N>(a, n_seqs, stream);
-    case 3: return piece_walk_go<3, CHANNEL, WITH_N>(a, n_seqs, stream);
-    case 4: return piece_walk_go<4, CHANNEL, WITH_N>(a, n_seqs, stream);
-    case 6: return piece_walk_go<6, CHANNEL, WITH_N>(a, n_seqs, stream);
-    default: return piece_walk_go<8, CHANNEL, WITH_N>(a, n_seqs, stream);
+    case 1: return piece_walk_go<1, CHANNEL, WITH_N>(a, stream);
+    case 2: return piece_walk_go<2, CHANNEL, WITH_N>(a, stream);
+    case 3: return piece_walk_go<3, CHANNEL, WITH_N>(a, stream);
+    case 4: return piece_walk_go<4, CHANNEL, WITH_N>(a, stream);
+    case 6: return piece_walk_go<6, CHANNEL, WITH_N>(a, stream);
+    default: return piece_walk_go<8, CHANNEL, WITH_N>(a, stream);
   }
 }

@@ -1033,31 +1033,69 @@ def attention_stream_status() -> int:
 # ---------------------------------------------------------------------------
 # the matrix-memory recurrence, attention over a cached latent, routed experts
 
-PIECE_MIN_TOKENS = 64            # tokens per sequence (on average) from which a step walks a recurrence in pieces ...
-PIECE_SHORTEST = 32              # ... none shorter than this, of one length for all sequences: the shortest that makes no more
-PIECE_CTAS = 296                 # blocks than two per processor, which all run at once
+PIECE_MIN_TOKENS = 64            # tokens per sequence (on average) from which a step may walk a recurrence in pieces ...
+PIECE_SHORTEST = 32              # ... none shorter than this
+
+
+def _pieces_pay(ctx, D: int, blocks: int, enough: int) -> bool:
+    """Whether the pieces' three kernels are faster than the one that walks every sequence from its start: long sequences, or
+    `enough` tokens of all `blocks` (a head's 128 columns each).  us of a mixer of width 1024 to 2048, in order -> in pieces: gated linear attention, 8 and 16 heads of
+    128 x 128, 128 tokens 54 -> 56, 58 -> 60, 160 tokens 61 -> 56, 68 -> 66, 4 sequences of 100 84 -> 70, 121 -> 97, 16 of 64
+    122 -> 97, 244 -> 127; matrix memory, 4 and 8 heads of 128 x 256, 128 tokens 39 -> 45, 52 -> 50, 200 tokens 54 -> 47, 70 -> 68,
+    4 of 100 56 -> 62, 92 -> 80, 16 of 64 94 -> 71, 179 -> 115; 4 heads of 256 x 256 160 tokens 70 -> 80, 200 tokens 81 -> 78."""
+    return ctx.n_tokens * blocks >= enough or ctx.n_tokens >= (160 if D <= 128 else 192) * ctx.n_seqs
 
 
 def _walks_pieces(ctx, D: int, V: int) -> bool:
-    """Whether a step's recurrence is walked in pieces side by side (csrc/piece_walk.cuh)."""
+    """Whether a step's recurrence can be walked in pieces side by side (csrc/piece_walk.cuh)."""
     return (not ctx.is_decode and ctx.n_tokens >= PIECE_MIN_TOKENS * ctx.n_seqs and V % 4 == 0
-            and D in (32, 64, 96, 128, 192, 256) and ctx.n_seqs * 256 <= 65535)
+            and D in (32, 64, 96, 128, 192, 256) and ctx.host_q_lens is not None and ctx.n_seqs <= 32767)
+
+
+def _piece_plan(ctx, room: int):
+    """(tokens per piece, pieces of all sequences, pieces of the sequences that have more than one), planned once per step: one
+    length for all sequences, the shortest whose pieces run at once, `room` of them, or in two rounds where those cost a tenth
+    less (8 sequences of 2,000 to 3,750 tokens, room for 18: 1 x 1,632 or 2 x 704 tokens, 2,101 -> 1,880 us).  A
+    sequence much shorter than a piece (a row of one token beside a prompt) holds its place for a part of that time and
+    counts for that part."""
+    key = ("pieces", room)
+    plan = ctx.extras.get(key)
+    if plan is None:
+        lens = [n for n in ctx.host_q_lens if n]
+        longest = max(lens, default=1)
+
+        def taken(length):           # (falls as the length grows)
+            return sum(n / length if 4 * n <= length else -(-n // length) for n in lens)
+
+        def shortest(room):
+            lo, hi = PIECE_SHORTEST // 8, max(-(-longest // 8), PIECE_SHORTEST // 8)
+            while lo < hi:           # at `hi` every sequence is one piece, whatever that takes
+                mid = (lo + hi) // 2
+                if taken(8 * mid) <= room:
+                    hi = mid
+                else:
+                    lo = mid + 1
+            return 8 * lo
+
+        def cost(length, rounds):    # operations per number of the state: walk 3 per token, a piece's own state 2, moving it
+            return rounds * ((3 if length >= longest else 5) * length + 120)
+        length, half = shortest(room), shortest(2 * room)
+        if cost(half, 2) < 0.9 * cost(length, 1):
+            length = half
+        pieces = [-(-n // length) for n in lens]
+        plan = ctx.extras[key] = (length, max(sum(pieces), 1), sum(n for n in pieces if n > 1))
+    return plan
 
 
 def _piece_scratch(ctx, H: int, D: int, width: int, prods: int, device):
-    """(tokens per piece, pieces of the longest sequence, what each leaves [n_seqs, H, pieces, D, width], its product of
-    decays [.., prods]); the scratch None where every sequence is one piece."""
-    room = PIECE_CTAS // (H * -(-width // 128))          # pieces of all sequences together that run at once
-    longest = max(ctx.host_q_lens)
-    length = max(PIECE_SHORTEST, -(-longest // 2048) * 8)      # (no more than 256 pieces)
-    while length < longest and sum(-(-n // length) for n in ctx.host_q_lens) > max(room, ctx.n_seqs):
-        length += 8
-    pieces = -(-longest // length)
-    if pieces == 1:
-        return length, 1, None, None
-    n = ctx.n_seqs * H * pieces
-    return (length, pieces, torch.empty(n * D * width, dtype=torch.float32, device=device),
-            torch.empty(n * prods, dtype=torch.float32, device=device))
+    """(tokens per piece, pieces, pieces that leave something, what each of those leaves [.., H, D, width], its product of decays
+    [.., H, prods]); the scratch None where every sequence is one piece.  Two blocks per processor run at once, one for D > 128."""
+    room = (2 if D <= 128 else 1) * _sm_count(device) // (H * -(-width // 128))
+    length, items, kept = _piece_plan(ctx, room)
+    if not kept:
+        return length, items, 0, None, None
+    return (length, items, kept, torch.empty(kept * H * D * width, dtype=torch.float32, device=device),
+            torch.empty(kept * H * prods, dtype=torch.float32, device=device))
 
 
 def mlstm_state_row(D: int, V: int) -> int:
@@ -1095,13 +1133,13 @@ def mlstm_step(proj, offsets, bias_i, bias_f, state, ctx, H, D, V, cap, qscale, 
     _i32(ctx.tok_seq, T, "tok_seq")
     coef = torch.empty((T, H, 3), dtype=torch.float32, device=proj.device)
     o_raw = torch.empty((T, H, V + 1), dtype=torch.float32, device=proj.device)
-    if not in_order and _walks_pieces(ctx, D, V) and not (off_q | off_k | off_v | ld) % 4 and not (proj.data_ptr() | state.data_ptr()) % 16:
-        length, pieces, local, prod = _piece_scratch(ctx, H, D, V + 4, 1, proj.device)
+    if not in_order and _walks_pieces(ctx, D, V) and _pieces_pay(ctx, D, H * -(-(V + 4) // 128), 6000) and not (off_q | off_k | off_v | ld) % 4 and not (proj.data_ptr() | state.data_ptr()) % 16:
+        *cut, local, prod = _piece_scratch(ctx, H, D, V + 4, 1, proj.device)
         _check(_lib("mlstm").ab_mlstm_prompt(
             _p(proj), ld, off_q, off_k, off_v, off_g, off_i, off_f, _p(bias_i), _p(bias_f), _p(state), row, H, D, V,
             _p(ctx.cu_q), _p(ctx.slots), _p(ctx.tok_seq), B, T, ctypes.c_float(cap), ctypes.c_float(qscale), _p(coef),
-            _p(o_raw), _p(norm_weight), ctypes.c_float(eps), _p(out), _dt(out), 1 if write_state else 0, pieces, length,
-            _p(local), _p(prod), _stream()), "mlstm_step", kernels=5 if pieces > 1 else 3)
+            _p(o_raw), _p(norm_weight), ctypes.c_float(eps), _p(out), _dt(out), 1 if write_state else 0, *cut,
+            _p(local), _p(prod), _stream()), "mlstm_step", kernels=3 if local is None else 5)
         return out
     _check(_lib("mlstm").ab_mlstm_step(
         _p(proj), ld, off_q, off_k, off_v, off_g, off_i, off_f, _p(bias_i), _p(bias_f), _p(state), row, H, D, V,
@@ -2019,13 +2057,13 @@ def gated_recurrence(mode, q, k, v, state, out, ctx, H, Hk, D, V, qscale=1.0, de
         ldd, dvec, dsc = 0, None, decay
     _i32(ctx.cu_q, ctx.n_seqs + 1, "cu_q")
     _i32(ctx.slots, ctx.n_seqs, "slots")
-    if (mode == "channel" and H == Hk and not in_order and _walks_pieces(ctx, D, V) and not (ldq | ldk | ldv | ldd) % 4
+    if (mode == "channel" and H == Hk and not in_order and _walks_pieces(ctx, D, V) and _pieces_pay(ctx, D, H * -(-V // 128), 3072) and not (ldq | ldk | ldv | ldd) % 4
             and not (q.data_ptr() | k.data_ptr() | v.data_ptr() | decay.data_ptr() | state.data_ptr()) % 16):
-        length, pieces, local, prod = _piece_scratch(ctx, H, D, V, D, q.device)
+        *cut, local, prod = _piece_scratch(ctx, H, D, V, D, q.device)
         _check(_lib("gated_recurrence").ab_gla_prompt(
             _p(q), ldq, _p(k), ldk, _p(v), ldv, _p(dvec), ldd, ctypes.c_float(qscale), _p(state), _p(out), _p(ctx.cu_q),
-            _p(ctx.slots), ctx.n_seqs, H, D, V, 1 if write_state else 0, pieces, length, _p(local), _p(prod),
-            _stream()), "gated_recurrence", kernels=3 if pieces > 1 else 1)
+            _p(ctx.slots), ctx.n_seqs, H, D, V, 1 if write_state else 0, *cut, _p(local), _p(prod),
+            _stream()), "gated_recurrence", kernels=1 if local is None else 3)
         return out
     cols = _recurrence_cols(ctx.n_seqs, H, V)
     _check(_lib("gated_recurrence").ab_gated_recurrence(

@@ -539,3 +539,39 @@ def test_float32_prompt_does_not_depend_on_the_step(mixer):
         for before, after in ((0, 0), (0, 900), (70, 0), (1, 450)):
             rows, s = run(before, cut, after)
             assert torch.equal(rows, want) and torch.equal(s, state), (cut, before, after)
+
+
+@pytest.mark.parametrize("D,V", [(32, 4), (128, 132), (192, 36), (256, 64)])
+@pytest.mark.parametrize("lens", [(1,) * 9 + (700,), (700,) + (1,) * 9, (30,) * 39 + (3000, 2, 500), (40, 900, 33, 64, 65, 1500)])
+def test_walk_in_pieces_of_ragged_steps(D, V, lens):
+    """Long sequences beside many short ones, sequences past the first 32: against the walk in the tokens' order.  Bound: both
+    walks' (`test_walk_in_pieces`), over the same walk of absolute values."""
+    from alpacca_b200 import ops
+    from alpacca_b200.parts.base import StateSpec
+    g = torch.Generator(device="cuda").manual_seed(D + len(lens))
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")        # noqa: E731
+    H, T = 2, sum(lens)
+    q, k, v = rnd(T, H * D), rnd(T, H * D), rnd(T, H * V)
+    a = torch.rand((T, H * D), generator=g, device="cuda") ** 0.1
+    hs = PartHarness([StateSpec((H, D, V))], "float32", max_tokens=8192, max_slots=48, max_positions=4096)
+    slots = [hs.cache.alloc_slot() for _ in lens]
+    ctx = hs.step(list(zip(slots, lens)))
+    assert ops._walks_pieces(ctx, D, V)
+    length, items, kept, local, prod = ops._piece_scratch(ctx, H, D, V, D, "cuda")
+    assert kept >= 2 and local.numel() == kept * H * D * V and items < len(lens) + kept
+    state = hs.cache.entry_view(0, ctx.block_tables).state
+    state.copy_(rnd(*state.shape))
+
+    def walk(state, q, k, v, **more):
+        state, out = state.clone(), torch.empty((T, H * V), device="cuda")
+        ops.gated_recurrence("channel", q, k, v, state, out, ctx, H, H, D, V, qscale=0.25, decay=a, **more)
+        return out, state
+    got, want = walk(state, q, k, v), walk(state, q, k, v, in_order=True)
+    size = walk(state.abs(), q.abs(), k.abs(), v.abs(), in_order=True)
+    at = 0
+    for slot, n in zip(slots, lens):
+        eps = 2 * (2 * torch.arange(1, n + 1, device="cuda")[:, None] + D + 4) * 2.0 ** -24
+        rows = slice(at, at + n)
+        assert ((got[0][rows] - want[0][rows]).abs() <= eps * size[0][rows]).all(), (slot, n)
+        assert ((got[1][slot] - want[1][slot]).abs() <= eps[-1] * size[1][slot]).all(), (slot, n)
+        at += n

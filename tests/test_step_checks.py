@@ -47,3 +47,33 @@ def test_an_engine_cannot_have_more_positions_than_its_model_was_built_for():
     assert Engine(model, max_tokens=256, max_slots=2, max_positions=64).max_positions == 64
     with pytest.raises(ValueError, match="built\\s+for 128"):
         Engine(model, max_tokens=256, max_slots=2, max_positions=129)
+
+
+@pytest.mark.parametrize("room,lens", [(12, [8192] + [1] * 11), (18, [1] * 17 + [2048]), (12, [4000] + [300] * 6), (12, [2048]), (1, [500]),
+                                       (18, [1500, 1000]), (296, [60000] + [1] * 99), (0, [5000, 3]), (12, [32768] * 8), (5, [1]),
+                                       (40, [100] * 39 + [3000]), (37, [2000 + 250 * i for i in range(8)])])
+def test_pieces_of_a_recurrent_prompt(room, lens):
+    """One length for all sequences, a multiple of 8; what has more than one piece fits beside the others; the shortest such
+    length; a long sequence is cut however many short ones stand beside it."""
+    from alpacca_b200 import ops
+    ctx = SimpleNamespace(host_q_lens=lens, extras={})
+    length, items, kept = ops._piece_plan(ctx, room)
+    pieces = [-(-n // length) for n in lens]
+    assert length % 8 == 0 and length >= 32 and items == sum(pieces) and kept == sum(p for p in pieces if p > 1)
+
+    def shortest(room):
+        fits = (n for n in range(32, max(lens) + 8, 8)
+                if sum(q / n if 4 * q <= n else -(-q // n) for q in lens) <= room)
+        return next(fits, max(-(-max(lens) // 8) * 8, 32))
+    one, two = shortest(room), shortest(2 * room)
+    two_rounds = 2 * (5 * two + 120) < 0.9 * ((3 if one >= max(lens) else 5) * one + 120)
+    assert length == (two if two_rounds else one) and kept <= 2 * room
+    if room >= 12 and 4 * sum(lens) < 5 * max(lens):
+        assert -(-max(lens) // length) >= room // 2
+    assert ops._piece_plan(ctx, room) is ctx.extras["pieces", room]
+
+
+def test_a_context_without_lengths_on_the_host_walks_in_order():
+    from alpacca_b200 import ops
+    ctx = SimpleNamespace(is_decode=False, n_tokens=500, n_seqs=1, host_q_lens=None, extras={})
+    assert not ops._walks_pieces(ctx, 128, 128)
