@@ -682,20 +682,33 @@ def _attention_decode_mma(qkv, out, cache, ctx, H, K, D, scale, window, rot=None
 PAIR_TC = True                   # plain scores and head size 128: the kernel with two query tiles per CTA (`_pair_pays`)
 
 
-def _pair_pays(n_ctas: int, max_kv_len: int, device) -> bool:
-    """Whether the kernel with two query tiles per CTA is the faster one: with most processors busy, in one round (short
-    prompts leave it a second one that is nearly empty) or over long keys.  us, one tile -> two: 128 CTAs of 1,024 keys 25.9 ->
-    24.2, 480 of 1,111 62 -> 74, 256 of 1,800 47 -> 51, 256 of 2,048 49 -> 45, 504 of 4,000 156 -> 139, 88 of 2,700 60 -> 53,
-    64 of 4,000 71 -> 73."""
-    return n_ctas >= 80 and (n_ctas <= _sm_count(device) or max_kv_len >= 2000)
+def _pair_pays(q_lens, kv_lens, H: int, K: int, sms: int) -> bool:
+    """Whether the kernel with two query tiles per CTA is the faster one.  us, one tile -> two, 32 query heads on 8 (on 32):
+    - up to 80 CTAs of two tiles the other kernel's CTAs, twice as many, have an SM each: 64 of 1,500 keys 29.7 -> 32.1;
+    - all of them in one round, from 432 keys per SM on: 88 CTAs of up to 700 keys 16.9 -> 18.8, 80 of 1,140 24.6 -> 26.0, of
+      1,640 34.9 -> 34.1, 112 of 896 21.9 -> 21.4, 128 of 256 11.3 -> 12.5, of 1,024 25.3 -> 23.8 (26.2 -> 25.9), of 2,256 52.4 ->
+      46.6 (66.7 -> 52.0);
+    - more, in several rounds, over long keys: 256 of 2,048 49.3 -> 44.9, 352 of them 300 tokens beside 200 on 3,000 held ones 63 -> 60
+      (84 -> 63), 520 of 500 beside 64 on 4,000 102 -> 74 (111 -> 80); 480 of 1,111 62 -> 74; but not where the other kernel needs
+      one round: 160 CTAs of 2,288 keys 52.2 -> 83.5."""
+    per_tile = 128 // (H // K)
+    ctas = K * sum(-(-n // (2 * per_tile)) for n in q_lens)
+    if ctas < 80:
+        return False
+    if ctas <= sms:
+        return K * sum(n * (kv - n / 2) for n, kv in zip(q_lens, kv_lens)) >= 432 * sms * 2 * per_tile
+    return max(kv_lens) >= 2000 and K * sum(-(-n // per_tile) for n in q_lens) > 2 * sms
 
 
 def _attention_prefill_tc(q, row_heads, out, k_pages, v_pages, table, ctx, H, K, D, scale, window, sink=None, score=(0,)):
     """Attention of a prompt step on the tcgen05 kernels: q [T, row_heads * D] whose rows start with the H query heads."""
     T, G = ctx.n_tokens, H // K
     if PAIR_TC and not score[0] and D == 128:
-        ctas = K * sum(-(-n // (2 * (128 // G))) for n in ctx.host_q_lens)
-        if _pair_pays(ctas, ctx.max_kv_len, q.device):
+        pays = ctx.extras.get(("attention_pair", H, K))
+        if pays is None:
+            pays = ctx.extras[("attention_pair", H, K)] = _pair_pays(ctx.host_q_lens, ctx.host_kv_lens, H, K,
+                                                                     _sm_count(q.device))
+        if pays:
             tile_seq, tile_q0, n_tiles, _ = _prefill_tiles(ctx, G, q.device, rows=128, together=2)
             _tc_unchecked["attention_pair_tc"] = True
             _check(_lib("attention_pair_tc").ab_attention_pair_tc(

@@ -77,3 +77,14 @@ def test_a_context_without_lengths_on_the_host_walks_in_order():
     from alpacca_b200 import ops
     ctx = SimpleNamespace(is_decode=False, n_tokens=500, n_seqs=1, host_q_lens=None, extras={})
     assert not ops._walks_pieces(ctx, 128, 128)
+
+
+@pytest.mark.parametrize("H,K,seqs,pays", [
+    (32, 8, [(0, 1024)], True), (32, 8, [(0, 700)], False), (32, 8, [(2000, 1000)], True), (32, 8, [(0, 512)] * 2, False),
+    (32, 8, [(500, 160)] * 4, False), (32, 8, [(2000, 160)] * 4, True), (32, 32, [(500, 192)] * 4, False), (32, 32, [(2000, 192)] * 4, True),
+    (32, 8, [(4000, 500)], False), (32, 8, [(0, 8192)], True), (32, 8, [(2000, 288)] * 4, False), (32, 8, [(2000, 320)] * 4, True),
+    (32, 8, [(4000, 64)] + [(0, 500)] * 8, True), (32, 8, [(0, 1111)] * 3, False), (32, 2, [(0, 4096)], True), (32, 8, [(0, 1)], False)])
+def test_which_prompts_take_two_query_tiles_per_block(H, K, seqs, pays):
+    """On 148 processors; the sides that were measured (held and new tokens of each sequence)."""
+    from alpacca_b200 import ops
+    assert ops._pair_pays([n for _, n in seqs], [h + n for h, n in seqs], H, K, 148) is pays
