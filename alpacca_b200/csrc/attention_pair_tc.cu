@@ -291,14 +291,15 @@ AB_API int ab_attention_pair_tc_status() {
   return v;
 }
 
-// Arguments as ab_attention_prefill_tc_sink's; tile_seq / tile_q0: tiles of 2 * floor(128 / G) tokens (sequence, first packed
+// Arguments as ab_attention_prefill_tc_dist's without a change of the scores; tile_seq / tile_q0: tiles of 2 * floor(128 / G) tokens (sequence, first packed
 // token).  out 16-byte aligned.
 AB_API int ab_attention_pair_tc(const void* qkv, int row_heads, int n_tokens, void* out, const void* k_pages,
                                 const void* v_pages, int n_pages, const int* block_table, int table_width, const int* tok_pos,
                                 const int* cu_q, const int* tile_seq, const int* tile_q0, int n_tiles, int H, int K, int D,
                                 float scale, int window, const float* sink, cudaStream_t stream) {
   if (n_tiles <= 0) return AB_OK;
-  if (D != 128 || K <= 0 || H % K || H / K > AP_ROWS || (long long)n_tiles * K > 0x7fffffffLL || row_heads < H)
+  if (D != 128 || K <= 0 || H % K || H / K > AP_ROWS || (long long)n_tiles * K > 0x7fffffffLL || row_heads < H ||
+      ((uintptr_t)out & 15))
     return AB_BAD_ARG;
   AtEncodeFn enc = at_encode_fn();
   int* status = ap_status_word();

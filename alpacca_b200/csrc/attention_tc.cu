@@ -472,22 +472,3 @@ AB_API int ab_attention_prefill_tc_dist(const void* qkv, int row_heads, int n_to
   if (e != cudaSuccess) return AB_CUDA_ERR + (int)e;
   return ab_launch_status();
 }
-
-AB_API int ab_attention_prefill_tc_sink(const void* qkv, int row_heads, int n_tokens, void* out, const void* k_pages,
-                                        const void* v_pages, int n_pages, const int* block_table, int table_width,
-                                        const int* tok_pos, const int* cu_q, const int* tile_seq, const int* tile_q0,
-                                        int n_tiles, int H, int K, int D, float scale, int window, const float* sink,
-                                        cudaStream_t stream) {
-  return ab_attention_prefill_tc_dist(qkv, row_heads, n_tokens, out, k_pages, v_pages, n_pages, block_table, table_width,
-                                      tok_pos, cu_q, tile_seq, tile_q0, n_tiles, H, K, D, scale, window, sink, SCORE_PLAIN,
-                                      nullptr, 0.f, stream);
-}
-
-// qkv [n_tokens, (H+2K)*D]: q | k | v of a token side by side; no sink.
-AB_API int ab_attention_prefill_tc(const void* qkv, int n_tokens, void* out, const void* k_pages, const void* v_pages,
-                                   int n_pages, const int* block_table, int table_width, const int* tok_pos,
-                                   const int* cu_q, const int* tile_seq, const int* tile_q0, int n_tiles, int H,
-                                   int K, int D, float scale, int window, cudaStream_t stream) {
-  return ab_attention_prefill_tc_sink(qkv, H + 2 * K, n_tokens, out, k_pages, v_pages, n_pages, block_table, table_width,
-                                      tok_pos, cu_q, tile_seq, tile_q0, n_tiles, H, K, D, scale, window, nullptr, stream);
-}
