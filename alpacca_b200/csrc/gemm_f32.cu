@@ -42,23 +42,23 @@ __device__ __forceinline__ float pair_sum(unsigned long long v) {
   return __uint_as_float((unsigned)v) + __uint_as_float((unsigned)(v >> 32));
 }
 
-// R rows from row r0 (n_rows exist; the others become zeros) of k0 .. k0 + BK - 1 (zeros from kend on)
+// R rows from row r0 (n_rows exist; the others become zeros) of k0 .. k0 + BK - 1 (zeros from kend on).  A thread keeps its k
+// and steps from row to row: an addition per copy where rows are not 16-byte aligned and a copy is four bytes (a
+// division and a product of 64 bits per copy: 2,000 rows of 3000x1021 524 us, 454 with plain loads before, 359 now).
 template <int R, int T, bool VEC>
 __device__ __forceinline__ void stage_rows(float* dst, const float* src, int ld, int r0, int n_rows, int k0, int kend) {
-  if (VEC) {
-#pragma unroll 1
-    for (int c = threadIdx.x; c < R * (BK / 4); c += T) {
-      const int r = c / (BK / 4), k = (c % (BK / 4)) * 4;
-      const bool in = r0 + r < n_rows && k0 + k < kend;      // kend is a multiple of 4 here
-      cp_async16(dst + r * KP + k, in ? src + (size_t)(r0 + r) * ld + k0 + k : src, in ? 16 : 0);
-    }
-  } else {
-#pragma unroll 1
-    for (int c = threadIdx.x; c < R * BK; c += T) {
-      const int r = c / BK, k = c % BK;
-      const bool in = r0 + r < n_rows && k0 + k < kend;
-      cp_async4(dst + r * KP + k, in ? src + (size_t)(r0 + r) * ld + k0 + k : src, in ? 4 : 0);
-    }
+  constexpr int W = VEC ? 4 : 1, RS = T / (BK / W);      // floats per copy, rows between a thread's copies
+  static_assert(T % (BK / W) == 0 && (R % RS == 0 || R < RS), "whole rounds of copies");
+  const int r = threadIdx.x / (BK / W), k = threadIdx.x % (BK / W) * W;
+  if (R < RS && r >= R) return;
+  const bool k_in = k0 + k < kend;                       // VEC: kend is a multiple of 4
+  const float* p = src + (size_t)(r0 + r) * ld + k0 + k;
+  float* d = dst + r * KP + k;
+#pragma unroll 4
+  for (int i = 0; i < (R + RS - 1) / RS; ++i, p += (size_t)RS * ld, d += RS * KP) {
+    const bool in = k_in && r0 + r + i * RS < n_rows;
+    if (VEC) cp_async16(d, in ? p : src, in ? 16 : 0);
+    else cp_async4(d, in ? p : src, in ? 4 : 0);
   }
 }
 
@@ -138,6 +138,7 @@ gemm_f32_nt_kernel(const float* __restrict__ A, int lda, const float* __restrict
     const float* w_s = smem + (t % STAGES) * STAGE + (BM + tx) * KP;
 #pragma unroll
     for (int k = 0; k < BK; k += 4) {
+
       ulonglong2 a[TM], w[TN];
 #pragma unroll
       for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(a_s + i * NY * KP + k);

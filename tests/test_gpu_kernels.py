@@ -664,3 +664,16 @@ def test_gemm_tc_persistent_swiglu(M, F, K, pair):
     ops.gemm_tc(x, w, out, bias=bias, swiglu=True, swap=False, pair=pair)
     close(out, g / (1 + torch.exp(-g)) * u, "bfloat16", "persistent swiglu epilogue")
     assert ops.gemm_tc_status() == 0
+
+
+@pytest.mark.parametrize("K", [1, 3, 16, 17, 33, 48, 513, 1021])
+@pytest.mark.parametrize("M,N", [(5, 33), (20, 130), (70, 130), (200, 1100)])
+def test_gemm_f32_ragged_k(M, N, K):
+    """Last tiles of every fill, rows that are not 16-byte aligned, on every tile height.  Bound: as for the tiles' test."""
+    from alpacca_b200 import ops
+    a, w, bias = rnd(M, K, seed=1), rnd(N, K, seed=2), rnd(N, seed=3)
+    want = a.double() @ w.double().T + bias.double()
+    bound = 2.0 ** -22 * (a.double().norm(dim=1)[:, None] * w.double().norm(dim=1)[None] + bias.double().abs())
+    out = torch.full((M + 1, N), 7.0, device="cuda")
+    ops.gemm_f32(a, w, out, bias=bias, n_rows=M)
+    assert ((out[:M].double() - want).abs() <= bound).all() and (out[M] == 7.0).all()
