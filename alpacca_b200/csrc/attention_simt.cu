@@ -18,7 +18,12 @@
 
 #define KEYS 8      // keys that a warp takes at a time; the exchanges below are written for 8
 
-template <typename T, int DPL>
+__device__ __forceinline__ size_t key_place(const int* bt, int s, int K, int kh, int page_size, int D) {
+  return (((size_t)bt[s / page_size] * K + kh) * page_size + s % page_size) * D;
+}
+
+// WHOLE: pages hold a multiple of KEYS keys, so that a run of them lies in one page; others look up every key
+template <typename T, int DPL, bool WHOLE>
 __global__ void attention_simt_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out,
                                       const T* __restrict__ k_pages, const T* __restrict__ v_pages,
                                       const int* __restrict__ block_table, int table_width,
@@ -46,13 +51,14 @@ __global__ void attention_simt_kernel(const T* __restrict__ q, int q_stride, T* 
   const int* bt = block_table + (size_t)b * table_width;
   // KEYS keys at a time (a run starts at a multiple of KEYS, so it does not depend on where the walk began)
   for (int s0 = lo - lo % KEYS; s0 <= pos; s0 += KEYS) {
-    const size_t base = (((size_t)bt[s0 / page_size] * K + kh) * page_size + s0 % page_size) * D;
+    const size_t base = key_place(bt, s0, K, kh, page_size, D);
     const T *k_run = k_pages + base, *v_run = v_pages + base;
     float v[KEYS];
 #pragma unroll
     for (int i = 0; i < KEYS; ++i) {
-      // a run lies in one page (pages hold a multiple of KEYS); a key outside lo .. pos gets no weight
+      // a key outside lo .. pos gets no weight
       const T* kv = k_run + (size_t)i * D;
+      if constexpr (!WHOLE) kv = k_pages + key_place(bt, min(s0 + i, pos), K, kh, page_size, D);
       float part = 0.f;
 #pragma unroll
       for (int j = 0; j < DPL; ++j) {
@@ -91,6 +97,7 @@ __global__ void attention_simt_kernel(const T* __restrict__ q, int q_stride, T* 
     for (int i = 0; i < KEYS; ++i) {
       const float pi = __shfl_sync(0xffffffffu, p, 4 * i);
       if (s0 + i < lo || s0 + i > pos) continue;     // the same for the whole warp
+      if constexpr (!WHOLE) v_run = v_pages + key_place(bt, s0 + i, K, kh, page_size, D) - (size_t)i * D;
 #pragma unroll
       for (int j = 0; j < DPL; ++j) {
         const int d = lane + 32 * j;
@@ -114,8 +121,9 @@ static int launch(const void* q, int q_stride, void* out, const void* k_pages, c
   const long long warps = (long long)n_tokens * H;
   const int wpb = 4;
   const unsigned blocks = (unsigned)((warps + wpb - 1) / wpb);
+  const bool whole = page_size % KEYS == 0;
 #define AB_GO(DPL)                                                                                       \
-  attention_simt_kernel<T, DPL><<<blocks, wpb * 32, 0, stream>>>(                                        \
+  (whole ? attention_simt_kernel<T, DPL, true> : attention_simt_kernel<T, DPL, false>)<<<blocks, wpb * 32, 0, stream>>>(                                        \
       (const T*)q, q_stride, (T*)out, (const T*)k_pages, (const T*)v_pages, block_table, table_width,   \
       tok_pos, tok_seq, n_tokens, H, K, D, page_size, scale, window)
   if (D <= 32) AB_GO(1);
@@ -131,7 +139,7 @@ AB_API int ab_attention_simt(const void* q, int q_stride, void* out, int dtype, 
                              const int* tok_seq, int n_tokens, int H, int K, int D, int page_size, float scale,
                              int window, cudaStream_t stream) {
   if (n_tokens <= 0) return AB_OK;
-  if (D <= 0 || D > 256 || H <= 0 || K <= 0 || H % K || page_size % KEYS) return AB_BAD_ARG;
+  if (D <= 0 || D > 256 || H <= 0 || K <= 0 || H % K || page_size <= 0) return AB_BAD_ARG;
   if (dtype == AB_F32)
     return launch<float>(q, q_stride, out, k_pages, v_pages, block_table, table_width, tok_pos, tok_seq,
                          n_tokens, H, K, D, page_size, scale, window, stream);

@@ -677,3 +677,31 @@ def test_gemm_f32_ragged_k(M, N, K):
     out = torch.full((M + 1, N), 7.0, device="cuda")
     ops.gemm_f32(a, w, out, bias=bias, n_rows=M)
     assert ((out[:M].double() - want).abs() <= bound).all() and (out[M] == 7.0).all()
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("page", [1, 5, 8, 12, 20])
+@pytest.mark.parametrize("window", [0, 11])
+def test_attention_simt_any_page_size(dtype, page, window):
+    """Pages that hold no multiple of the eight keys that a warp takes at a time, and the smallest that do."""
+    from alpacca_b200 import ops
+    H, K, D, lengths, q_lens = 4, 2, 40, [37, 3, 60], [9, 3, 1]
+    table, kp, vp = make_paged(lengths, sum(-(-n // page) for n in lengths) + 2, K, D, DT[dtype], page=page, seed=page)
+    T = sum(q_lens)
+    qkv = rnd(T, (H + 2 * K) * D, dtype=DT[dtype], seed=3)
+    ks = [rnd(n, K, D, dtype=DT[dtype], seed=4 + b) for b, n in enumerate(lengths)]
+    vs = [rnd(n, K, D, dtype=DT[dtype], seed=8 + b) for b, n in enumerate(lengths)]
+    for b, n in enumerate(lengths):
+        for i in range(n):
+            where = int(table[b, i // page])
+            kp[where, :, i % page], vp[where, :, i % page] = ks[b][i], vs[b][i]
+    pos = torch.cat([torch.arange(n - q, n) for n, q in zip(lengths, q_lens)]).to(torch.int32).cuda()
+    seq = torch.cat([torch.full((q,), b) for b, q in enumerate(q_lens)]).to(torch.int32).cuda()
+    out = torch.zeros(T, H * D, dtype=DT[dtype], device="cuda")
+    ops.attention_simt(qkv, out, kp, vp, table, pos, seq, T, H, K, D, D ** -0.5, window)
+    q = qkv.double().cpu().view(T, H + 2 * K, D)[:, :H]
+    at = 0
+    for b, n in enumerate(q_lens):
+        want = ref_attention(q[at:at + n], ks[b].double().cpu(), vs[b].double().cpu(), pos[at:at + n].cpu(), D ** -0.5, window)
+        close(out[at:at + n].view(n, H, D), want, dtype, f"sequence {b}")
+        at += n
