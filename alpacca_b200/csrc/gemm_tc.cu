@@ -409,7 +409,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 #define TP_BN 256
 // BN columns per tile; fewer than 256 where tiles of 256 would leave most SMs without one (grouped form)
 template <int BN> struct TpShape {
-  static constexpr int STAGES = BN == 256 ? 4 : 6;
+  static constexpr int STAGES = BN == 256 ? 4 : BN == 128 ? 6 : 8;
   static constexpr int A_BYTES = TC_BM * TC_BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + BN * TC_BK * 2;
   static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 + 256;
@@ -433,14 +433,18 @@ __device__ __forceinline__ void tp_tile_origin(int tile, int tiles_m, int tiles_
 }
 
 // Warps that empty the accumulators.  The grouped form has two per 32 rows, each for every second 16 columns: it runs tiles
-// few per CTA, whose tail nothing hides
-#define TP_TAIL_WARPS(GROUPED) ((GROUPED) ? 8 : 4)
+// few per CTA, whose tail nothing hides.  GELU in its erf form has four on narrow tiles: 16,384 erff of a tile of 128 x 128 keep the
+// issue slots busy for longer than the product takes (feed-forward of width 1024, 8 ungated experts, two -> four, us: 33 tokens 22.4 ->
+// 21.4, 200 26.9 -> 26.2); on tiles of 256, several to a CTA, they disturb the next tile's products (16 experts at width 2048, 1,000
+// tokens 102 -> 116)
+#define TP_TAIL_WARPS(GROUPED, EPI, BN) \
+  (!(GROUPED) ? 4 : (BN) < 256 && ((EPI) == EPI_GELU_BF16 || (EPI) == EPI_GEGLU_BF16) ? 16 : 8)
 // GROUPED: the rows come in groups that start on tiles, each with a matrix of its own (routed experts): row tile i belongs
 // to group tile_group[i] and meets the rows group * N .. of W.  How many row tiles there are (*row_tiles, at most
 // tiles_m) is known on the device only, from kernels before this one; so everything waits for those.  Without tile_group every
 // group has group_tiles row tiles; with x_shared they are the same rows of X for all groups (few tokens: every expert for all).
 template <int EPI, bool GROUPED, int BN>
-__global__ void __launch_bounds__(64 + 32 * TP_TAIL_WARPS(GROUPED))
+__global__ void __launch_bounds__(64 + 32 * TP_TAIL_WARPS(GROUPED, EPI, BN))
 gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                           void* __restrict__ Y, const float* __restrict__ bias, int* __restrict__ status, int M, int N,
                           int K, int ldy, int tiles_m, int n_tiles, const int* __restrict__ tile_group,
@@ -474,7 +478,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < TP_STAGES; ++s) { mbar_init(full + s, 1); mbar_init(empty + s, 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(acc_full + b, 1); mbar_init(acc_empty + b, TP_TAIL_WARPS(GROUPED)); }
+    for (int b = 0; b < 2; ++b) { mbar_init(acc_full + b, 1); mbar_init(acc_empty + b, TP_TAIL_WARPS(GROUPED, EPI, BN)); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -563,7 +567,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
       float factor = 1.f;
       if (EPI == EPI_RELU2_BF16 && row_factor != nullptr && m0 + row < m_stop) factor = row_factor[m0 + row];
 #pragma unroll 1
-      for (int c0 = (warp - 2) / 4 * 16; c0 < BN; c0 += TP_TAIL_WARPS(GROUPED) * 4) {
+      for (int c0 = (warp - 2) / 4 * 16; c0 < BN; c0 += TP_TAIL_WARPS(GROUPED, EPI, BN) * 4) {
         float v[16];
         tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)buf * BN + c0, v);
         if (EPI == EPI_RELU2_BF16) relu2_16(v, factor);
@@ -935,7 +939,7 @@ AB_API int ab_gemm_tc_persistent(const void* X, const void* W, const float* bias
 // Rows in groups with a matrix each (see the kernel): Y [max_rows, ..] and X [max_rows, K] in row tiles of 128 (max_rows a
 // multiple of 128), W [groups * N, K]; tile_group int [max_rows / 128], row_tiles int [1] on the device.  Without those two
 // every group has max_rows / groups rows of which the first group_rows count (the others are not stored); with `x_shared` X is
-// [group_rows, K], the same for all groups.  `bn`: columns per tile, 128 or 256.  Epilogue kinds 0 (bfloat16), 1 (float32), 2 and 8 (SiLU or GELU on the gate), 6 and 7 (GELU,
+// [group_rows, K], the same for all groups.  `bn`: columns per tile, 64, 128 or 256.  Epilogue kinds 0 (bfloat16), 1 (float32), 2 and 8 (SiLU or GELU on the gate), 6 and 7 (GELU,
 // SiLU) and 5 (squared ReLU, of the products times row_factor [max_rows] where it is given).
 AB_API int ab_gemm_tc_grouped(const void* X, const void* W, void* Y, int max_rows, int N, int K, int groups, int ldy,
                               int epilogue_kind, const int* tile_group, const int* row_tiles, const float* row_factor,
@@ -955,7 +959,7 @@ AB_API int ab_gemm_tc_grouped(const void* X, const void* W, void* Y, int max_row
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   }
   const int tiles_m = max_rows / TC_BM, group_tiles = tile_group == nullptr ? tiles_m / groups : 1;
-  if (bn != 128 && bn != TP_BN) return AB_BAD_ARG;
+  if (bn != 64 && bn != 128 && bn != TP_BN) return AB_BAD_ARG;
   const int tiles_n = (N + bn - 1) / bn;
   CUtensorMap mx, mw;
   if (!make_map(&mx, X, x_shared ? group_rows : max_rows, K, TC_BM)) return AB_BAD_ARG;
@@ -968,13 +972,13 @@ AB_API int ab_gemm_tc_grouped(const void* X, const void* W, void* Y, int max_row
     cudaError_t e = cudaFuncSetAttribute(gemm_tc_persistent_kernel<E, true, BN>,                                   \
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, TpShape<BN>::SMEM);          \
     if (e != cudaSuccess) return AB_CUDA_ERR + (int)e;                                                             \
-    e = ab_launch(gemm_tc_persistent_kernel<E, true, BN>, dim3(grid), dim3(64 + 32 * TP_TAIL_WARPS(true)), (size_t)TpShape<BN>::SMEM, \
+    e = ab_launch(gemm_tc_persistent_kernel<E, true, BN>, dim3(grid), dim3(64 + 32 * TP_TAIL_WARPS(true, E, BN)), (size_t)TpShape<BN>::SMEM, \
                   stream, mx, mw, Y, (const float*)nullptr, status, max_rows, N, K, ldy, tiles_m, n_tiles,         \
                   tile_group, row_tiles, row_factor, group_tiles, x_shared, group_rows);                           \
     if (e != cudaSuccess) return AB_CUDA_ERR + (int)e;                                                             \
     return ab_launch_status();                                                                                     \
   }
-#define AB_GO(E) { if (bn == 128) AB_GO_BN(E, 128) else AB_GO_BN(E, TP_BN) }
+#define AB_GO(E) { if (bn == 64) AB_GO_BN(E, 64) else if (bn == 128) AB_GO_BN(E, 128) else AB_GO_BN(E, TP_BN) }
   switch (epilogue_kind) {
     case EPI_STORE_BF16: AB_GO(EPI_STORE_BF16)
     case EPI_STORE_F32: AB_GO(EPI_STORE_F32)

@@ -2273,24 +2273,35 @@ def row_dots(h, w, n_tokens):
 
 
 MOE_GEMV_MAX_ROWS = 32             # up to here the skinny products of csrc/moe_gemv.cu
-MOE_ALL_MAX_TILES = 2              # row tiles of 128 tokens up to which every expert may run for all tokens
+# pairs x ff x width up to which a step without a shared expert (whose sum is rounded once) reads rows once per pair: a cluster's
+# merge costs more than the few rows that tokens share.  us, skinny products -> pairs: 8 experts of 704, width 1024, 2 chosen, gated 1
+# token 13.3 -> 11.5, 4 tokens 18.1 -> 15.2, 6 tokens 19.1 -> 18.1, 7 tokens 19.5 -> 20.1, ungated 1 token 12.1 -> 10.3, 6 tokens 15.6 ->
+# 15.4; 16 experts of 1408, width 2048, 4 chosen, 1 token gated 28.3 -> 28.5, ungated 19.8 -> 22.8
+MOE_FEW_UNITS = 9 << 20
+MOE_ALL_MAX_TILES = 3              # row tiles of 128 tokens up to which every expert may run for all tokens
 
 
 def _all_experts_pay(per, n_tokens, top, n_experts, width, n_up, device):
     """Every expert for all tokens, or a plan: a chosen expert costs one row tile at least either way, so with one tile of tokens
-    and most experts chosen the plan (a sort and a copy of the rows) buys nothing.  With two it saves up to half of the tiles,
-    which shows once an SM has more than one tile of a product (B200, us, plan -> all, 200 tokens: 8 experts of 704, width
-    1024, gated 35 -> 31, ungated 36 -> 31; 16 experts of 1408, width 2048, gated 88 -> 96, ungated 74 -> 82)."""
+    and most experts chosen the plan (a count and a copy of the rows) buys nothing.  With two or three it saves tiles, which
+    shows once an SM has more than one tile of a product (B200, us, plan -> all, 200 tokens: 8 experts of 704, width
+    1024, gated 29.0 -> 25.7, ungated 29.4 -> 26.2; 16 experts of 1408, width 2048, gated 84.5 -> 90.7, ungated 68 -> 76; 300
+    tokens of width 1024: 29.6 -> 28.6, 29.6 -> 28.9)."""
     if per > MOE_ALL_MAX_TILES or n_tokens * top < 2 * n_experts:
         return False
     return per == 1 or per * n_experts * (-(-n_up // 256) + -(-width // 256)) <= 2 * _sm_count(device)
 
 
-def _grouped_columns(row_tiles, n, device):
-    """Columns of a tile of `gemm_tc_grouped`: 128 where the tiles of 256 would not even fill half of the SMs, so that twice as
-    many still run at once (B200, us of a whole feed-forward, 256 -> 128 columns of the first product: 24 tiles, 30.5 -> 26.7;
-    48 tiles, 22.8 -> 23.1; 69 tiles, 45.1 -> 41.5; 96 tiles, 57.5 -> 59.8; 117 tiles, 53.3 -> 55.5)."""
-    return 128 if 2 * row_tiles * -(-n // 256) <= _sm_count(device) else 256
+def _grouped_columns(row_tiles, n, device, planned=False):
+    """Columns of a tile of `gemm_tc_grouped`: the fewest whose tiles still run at once, one per SM: a tile of fewer columns has
+    less to bring and a shorter tail.  64 only behind a plan, whose row tiles are few; us of a whole feed-forward by columns of
+    the two products, width 1024, ungated: 200 tokens, all experts, 128,128 26.2, 64,64 29.2, 256,256 30; 512 tokens by plan 64,128
+    32.6, 128,128 33.4, 128,256 35; gated: 300 tokens, all experts 256,256 28.6, 256,128 30.2, 700 by plan 256,128 37.7, 128,128 41.2,
+    256,256 40.3.  (Width 2048, 16 experts: 256 columns are 176 tiles; 128 measured within 3 %.)"""
+    for columns in (64, 128) if planned else (128,):
+        if row_tiles * -(-n // columns) <= _sm_count(device):
+            return columns
+    return 256
 
 
 GROUPED_TAILS = {None: 0, "relu2": 5, "gelu": 6, "silu": 7}       # on a product without a gate ...
@@ -2305,7 +2316,7 @@ def gemm_tc_grouped(x, w, out, n_groups, tile_group, row_tiles, gated=False, act
     multiplied by its row's number of row_factor (float32 [R]) if that is given.  All bfloat16, but `out` may be float32 where
     there is no activation.
     Without `tile_group` and `row_tiles` every group has R / n_groups rows of which the first `group_rows` count (the others are
-    left alone); `x` is then [R, K], or [group_rows, K] for the same rows in all groups.  `columns` of a tile: 128 or 256."""
+    left alone); `x` is then [R, K], or [group_rows, K] for the same rows in all groups.  `columns` of a tile: 64, 128 or 256."""
     _cuda(x, w, out, tile_group, row_tiles, row_factor)
     _need(act in (GROUPED_GATED_TAILS if gated else GROUPED_TAILS), f"gemm_tc_grouped: activation {act!r}")
     f32 = out.dtype == torch.float32
@@ -2344,9 +2355,9 @@ def moe_shared_experts(h, gate_up, down, n_experts, top, out, ctx, activation="s
     `table` int32 [vocab, top] with weight 1 / top each.  out [T, width] float32, or of h's dtype: the experts' outputs are
     then float32 until their sum is rounded once.
 
-    bfloat16: up to MOE_GEMV_MAX_ROWS tokens two skinny products that read the chosen experts' weights once; more tokens
-    grouped products over the (token, expert) pairs in order of their experts, the shared expert beside them as a dense
-    feed-forward.  Everything else (32-bit, widths that are no multiples of 8): a warp per (pair, unit)."""
+    bfloat16: a few pairs without a shared expert a warp per (pair, unit) (MOE_FEW_UNITS); up to MOE_GEMV_MAX_ROWS tokens two
+    skinny products that read the chosen experts' weights once; more tokens grouped products over the (token, expert) pairs in
+    order of their experts, the shared expert beside them as a dense feed-forward.  Everything else (32-bit, widths that are no multiples of 8): a warp per (pair, unit)."""
     idx, wts = choice if choice is not None else (None, None)
     gate_up_s, down_s = shared if shared is not None else (None, None)
     _cuda(h, gate_up, down, out, idx, wts, table, gate_logits, gate_up_s, down_s)
@@ -2400,10 +2411,10 @@ def moe_shared_experts(h, gate_up, down, n_experts, top, out, ctx, activation="s
             groups = (plan[:n_tiles], plan[n_tiles:])
         act = torch.empty((n_tiles * 128, ff), dtype=h.dtype, device=dev)
         gemm_tc_grouped(rows, gate_up, act, n_experts, *groups, gated=gated, act=activation, row_factor=row_w, group_rows=T,
-                        columns=_grouped_columns(tiles, rpu * ff, dev))
+                        columns=_grouped_columns(tiles, rpu * ff, dev, plan is not None))
         if plan is None or out.dtype != torch.float32:
             rows = torch.empty((n_tiles * 128, width), dtype=h.dtype if out.dtype == torch.float32 else torch.float32, device=dev)
-        gemm_tc_grouped(act, down, rows, n_experts, *groups, group_rows=T, columns=_grouped_columns(tiles, width, dev))
+        gemm_tc_grouped(act, down, rows, n_experts, *groups, group_rows=T, columns=_grouped_columns(tiles, width, dev, plan is not None))
         ys = None
         if shared is not None:
             act_s = torch.empty((T, fs), dtype=h.dtype, device=dev)
@@ -2421,7 +2432,8 @@ def moe_shared_experts(h, gate_up, down, n_experts, top, out, ctx, activation="s
                                           per * 128, _stream()), "moe_combine")
         return out
     act = torch.empty((max(T, 1), top * ff + fs), dtype=h.dtype, device=dev)
-    if fast and T <= MOE_GEMV_MAX_ROWS and n_experts <= 512 and top <= 32 and (gated or (ff % 16 == 0 and fs % 16 == 0)):
+    few = shared is None and out.dtype == h.dtype and T * top * ff * width <= MOE_FEW_UNITS
+    if fast and not few and T <= MOE_GEMV_MAX_ROWS and n_experts <= 512 and top <= 32 and (gated or (ff % 16 == 0 and fs % 16 == 0)):
         slabs, slices = -(-width // 16), 1
         while slices < 8 and slabs * slices * 4 < 3 * _sm_count(dev):
             slices *= 2
