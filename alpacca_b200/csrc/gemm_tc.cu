@@ -433,18 +433,16 @@ __device__ __forceinline__ void tp_tile_origin(int tile, int tiles_m, int tiles_
 }
 
 // Warps that empty the accumulators.  The grouped form has two per 32 rows, each for every second 16 columns: it runs tiles
-// few per CTA, whose tail nothing hides.  GELU in its erf form has four on narrow tiles: 16,384 erff of a tile of 128 x 128 keep the
-// issue slots busy for longer than the product takes (feed-forward of width 1024, 8 ungated experts, two -> four, us: 33 tokens 22.4 ->
-// 21.4, 200 26.9 -> 26.2); on tiles of 256, several to a CTA, they disturb the next tile's products (16 experts at width 2048, 1,000
-// tokens 102 -> 116)
-#define TP_TAIL_WARPS(GROUPED, EPI, BN) \
-  (!(GROUPED) ? 4 : (BN) < 256 && ((EPI) == EPI_GELU_BF16 || (EPI) == EPI_GEGLU_BF16) ? 16 : 8)
+// few per CTA, whose tail nothing hides.  GELU in its erf form has four: 16,384 erff of a tile of 128 x 128 keep the issue slots
+// busy for longer than the product takes (feed-forward of 8 ungated experts, width 1024, two -> four, us: 33 tokens 22.4 -> 21.4, 200
+// 26.9 -> 26.2; 16 experts, width 2048: 33 tokens 54.1 -> 52.3, 512 95.8 -> 94.2, 2,000 160.9 -> 160.4)
+#define TP_TAIL_WARPS(GROUPED, EPI) (!(GROUPED) ? 4 : (EPI) == EPI_GELU_BF16 || (EPI) == EPI_GEGLU_BF16 ? 16 : 8)
 // GROUPED: the rows come in groups that start on tiles, each with a matrix of its own (routed experts): row tile i belongs
 // to group tile_group[i] and meets the rows group * N .. of W.  How many row tiles there are (*row_tiles, at most
 // tiles_m) is known on the device only, from kernels before this one; so everything waits for those.  Without tile_group every
 // group has group_tiles row tiles; with x_shared they are the same rows of X for all groups (few tokens: every expert for all).
 template <int EPI, bool GROUPED, int BN>
-__global__ void __launch_bounds__(64 + 32 * TP_TAIL_WARPS(GROUPED, EPI, BN))
+__global__ void __launch_bounds__(64 + 32 * TP_TAIL_WARPS(GROUPED, EPI))
 gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                           void* __restrict__ Y, const float* __restrict__ bias, int* __restrict__ status, int M, int N,
                           int K, int ldy, int tiles_m, int n_tiles, const int* __restrict__ tile_group,
@@ -478,7 +476,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < TP_STAGES; ++s) { mbar_init(full + s, 1); mbar_init(empty + s, 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(acc_full + b, 1); mbar_init(acc_empty + b, TP_TAIL_WARPS(GROUPED, EPI, BN)); }
+    for (int b = 0; b < 2; ++b) { mbar_init(acc_full + b, 1); mbar_init(acc_empty + b, TP_TAIL_WARPS(GROUPED, EPI)); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -567,7 +565,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
       float factor = 1.f;
       if (EPI == EPI_RELU2_BF16 && row_factor != nullptr && m0 + row < m_stop) factor = row_factor[m0 + row];
 #pragma unroll 1
-      for (int c0 = (warp - 2) / 4 * 16; c0 < BN; c0 += TP_TAIL_WARPS(GROUPED, EPI, BN) * 4) {
+      for (int c0 = (warp - 2) / 4 * 16; c0 < BN; c0 += TP_TAIL_WARPS(GROUPED, EPI) * 4) {
         float v[16];
         tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)buf * BN + c0, v);
         if (EPI == EPI_RELU2_BF16) relu2_16(v, factor);
@@ -972,7 +970,7 @@ AB_API int ab_gemm_tc_grouped(const void* X, const void* W, void* Y, int max_row
     cudaError_t e = cudaFuncSetAttribute(gemm_tc_persistent_kernel<E, true, BN>,                                   \
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, TpShape<BN>::SMEM);          \
     if (e != cudaSuccess) return AB_CUDA_ERR + (int)e;                                                             \
-    e = ab_launch(gemm_tc_persistent_kernel<E, true, BN>, dim3(grid), dim3(64 + 32 * TP_TAIL_WARPS(true, E, BN)), (size_t)TpShape<BN>::SMEM, \
+    e = ab_launch(gemm_tc_persistent_kernel<E, true, BN>, dim3(grid), dim3(64 + 32 * TP_TAIL_WARPS(true, E)), (size_t)TpShape<BN>::SMEM, \
                   stream, mx, mw, Y, (const float*)nullptr, status, max_rows, N, K, ldy, tiles_m, n_tiles,         \
                   tile_group, row_tiles, row_factor, group_tiles, x_shared, group_rows);                           \
     if (e != cudaSuccess) return AB_CUDA_ERR + (int)e;                                                             \
