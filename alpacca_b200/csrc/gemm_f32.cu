@@ -1,65 +1,107 @@
-// C[M,N] = A[M,K] . W[N,K]^T (+ bias[N]) in true 32-bit: plain FMA on the CUDA
-// cores, no tensor-core mode of reduced precision anywhere.
+// C[M,N] = A[M,K] . W[N,K]^T (+ bias[N]) with the precision of 32-bit sums, on the tensor cores.
 //
-// The order of an output's sum depends on K alone: the k range is cut into up to GROUPS runs (of a
-// multiple of BK, at least SHORTEST); a run is two chains of fused multiply-adds in ascending order, one over
-// its even k and one over its odd k, added at its end; the runs are added in ascending order.  So a value does
-// not depend on M, on the tile it falls into, on whether the runs of a tile are computed by one CTA or by a cluster of CTAs, or on
-// what other rows are in the batch: the same token gives the same bits alone and in any batch.  This is the
-// matrix product of the 32-bit path (the reference's float32 path uses BLAS SGEMM, alpacca/tensor.py:91-97).
+// Every 32-bit number is split into three bfloat16 numbers that add up to it exactly (x = h + m + l: h is x rounded,
+// m the rest rounded, l what is then left, at most eight bits).  A product needs six of the nine partial products,
+//   a w = ah wh + (ah wm + am wh) + (ah wl + am wm + al wh)        the other three are below 2^-26 of |a w|,
+// each exact in 32 bits, summed by tcgen05.mma in three 32-bit accumulators in tensor memory, one per bracket.  The sums
+// of the tensor cores cut off instead of rounding, so the leading accumulator holds 32 k only: adding warps then add it to
+// a rounded 32-bit sum in registers.  The two others are 2^-8 smaller and run to the end of a run of k.
+// Error against 64 bits, root mean square over |a| |w| (before: multiply-adds in 32 bits): normal numbers 2.0e-9 at 2,048 k
+// (4.7e-9), 1.4e-9 at 8,192 (4.5e-9), 5.6e-9 at 128 (1.3e-8); all of one sign 4.2e-8 at 2,048 (4.7e-8).  A layer of the 1B
+// shape 2.5e-7 (5.4e-7).
 //
-// What bounds it: the FMA pipes (128 multiply-adds per clock and SM, 74 TFLOP/s) for many rows, HBM (the
-// weights) for few.  Two k of an output side by side in a register pair are one fma.rn.f32x2, whose operands
-// come out of 16-byte shared loads without packing, so half the issue slots are free for the loads.  Rows
-// stay [row][k] in shared memory (cp.async, no transposition), BK + 4 floats apart: eight neighbouring
-// threads read eight rows without a bank conflict.  It reaches 46 TFLOP/s (2,048 rows of
-// 16384x2048: 5.4 -> 3.0 ms); two fma.rn.f32 in place of the pair measured the same, so the shared loads bind, not
-// the FMA pipes.  333 rows of q|k|v, o, gate|up and down of the 1B shape: 216 -> 123, 215 -> 87, 1055 -> 573,
-// 866 -> 312 us; one row: 116 -> 11, 116 -> 11, 212 -> 38, 461 -> 33 us (3.6 TB/s on gate|up).
+// The order of an output's sum depends on K alone: the k range is cut into up to GROUPS runs (of a multiple of BK, at
+// least SHORTEST), a run into stages of 32; the first four runs are added in ascending order, the others too, then both.  So a value does not depend on M, on
+// the tile it falls into, on whether the runs of a tile are computed by one CTA or by a cluster of CTAs, or on what other
+// rows are in the batch: the same token gives the same bits alone and in any batch.  This is the matrix product of the
+// 32-bit path (the reference's float32 path uses BLAS SGEMM, alpacca/tensor.py:91-97).
+//
+// A number that is not finite, or above the largest bfloat16, splits into infinities and NaNs; so do the sums.  An
+// output that comes out not finite is therefore formed again by plain multiply-adds (`plain_dot`): what the sum gives
+// in 32 bits, infinities included.
+//
+// A tile is 128 rows of W (the 128 rows of an MMA) by n <= 128 rows of A.  Splitting warps bring both operands' 32-bit rows
+// by cp.async into a ring in shared memory (each thread only what it splits itself, so nobody waits for anybody), split
+// them and store the parts in the swizzled form that the MMA reads; adding warps move the leading accumulator; one lane of
+// another warp issues the MMAs, four per 16 k: [wm|wl] and [wh|wm] lie side by side, so that two MMAs do the work of four.
+// What bounds it: for many rows the splitting and adding instructions (some 1,400 clocks a stage at n = 128, the tensor cores
+// 768); for few rows the latency of a stage, hidden by two CTAs per processor, and HBM.
+// us before (multiply-adds) / now: 333 rows of q|k|v, o, gate|up and down of the 1B shape 123 / 44, 87 / 44, 570 / 261,
+// 316 / 154; 64 rows 34 / 25, 24 / 24, 114 / 61, 81 / 62; 17 rows 22 / 17, 15 / 15, 67 / 52, 50 / 45; one row 11.6 / 12.2,
+// 10.8 / 11.1, 35.8 / 33.6, 35.5 / 31.7.  2,048 rows of 16384x2048: 2,960 / 1,242 (111 TFLOP/s, 46 before).
+// Tried: 16 warps that split and add in turn (333 rows of gate|up 243, one row of q|k|v 15.8); rounding in integers in place of the
+// conversion instruction (the same); two leading accumulators (one row 0.8 us slower a product).
+//
+// Every wait on an mbarrier is bounded; a thread that gives up leaves a code in `gemm_f32_stuck`, all roles fall through
+// to the end, where TMEM is given back, and the outputs are NaN until `plain_dot` has formed them.
+#include "attention_tc.cuh"
 #include "common.cuh"
 #include "launch.cuh"
 
-#define BK 32
-#define KP (BK + 4)      // floats from row to row in shared memory
+#define BK 32            // k of a stage: 64 bytes of a split row, the width of the swizzle
 #define GROUPS 8         // runs of k; also the CTAs of a cluster that share a tile
-#define SHORTEST 128     // a run's k at least: adding up runs of 32 was a fifth of a product over 128 k
-#define STAGES 2         // two of four CTAs per SM hide the copies: a third stage, three CTAs per SM, was 0 to 10 % slower
+#define SHORTEST 128     // a run's k at least
+#define EARLY 256        // k of W that are fetched to the L2 before the kernel before this one has ended
+#define W_PART (128 * 64)          // bytes of one part of the weights' rows in a stage
 
-__device__ __forceinline__ void cp_async16(float* dst, const float* src, int bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
-               "r"(bytes));
-}
-__device__ __forceinline__ void cp_async4(float* dst, const float* src, int bytes) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
-               "r"(bytes));
-}
-__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-  unsigned long long d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ float pair_sum(unsigned long long v) {
-  return __uint_as_float((unsigned)v) + __uint_as_float((unsigned)(v >> 32));
-}
+__device__ int gemm_f32_stuck;     // 0, or the code of a wait that was given up
 
-// R rows from row r0 (n_rows exist; the others become zeros) of k0 .. k0 + BK - 1 (zeros from kend on).  A thread keeps its k
-// and steps from row to row: an addition per copy where rows are not 16-byte aligned and a copy is four bytes (a
-// division and a product of 64 bits per copy: 2,000 rows of 3000x1021 524 us, 454 with plain loads before, 359 now).
-template <int R, int T, bool VEC>
-__device__ __forceinline__ void stage_rows(float* dst, const float* src, int ld, int r0, int n_rows, int k0, int kend) {
-  constexpr int W = VEC ? 4 : 1, RS = T / (BK / W);      // floats per copy, rows between a thread's copies
-  static_assert(T % (BK / W) == 0 && (R % RS == 0 || R < RS), "whole rounds of copies");
-  const int r = threadIdx.x / (BK / W), k = threadIdx.x % (BK / W) * W;
-  if (R < RS && r >= R) return;
-  const bool k_in = k0 + k < kend;                       // VEC: kend is a multiple of 4
-  const float* p = src + (size_t)(r0 + r) * ld + k0 + k;
-  float* d = dst + r * KP + k;
-#pragma unroll 4
-  for (int i = 0; i < (R + RS - 1) / RS; ++i, p += (size_t)RS * ld, d += RS * KP) {
-    const bool in = k_in && r0 + r + i * RS < n_rows;
-    if (VEC) cp_async16(d, in ? p : src, in ? 16 : 0);
-    else cp_async4(d, in ? p : src, in ? 4 : 0);
-  }
+__device__ __forceinline__ void cp_async16(uint32_t dst, const float* src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes));
+}
+__device__ __forceinline__ void cp_async4(uint32_t dst, const float* src, int bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes));
+}
+// A product of K-major operand rows of 64 bytes with the 64-byte swizzle (groups of 8 rows are 512 bytes apart), by the
+// lower words of their descriptors: the upper ones are the same, and one thread issues all of them, so every
+// instruction around them counts.
+#define SPLIT_DESC_LO(addr) (((addr) >> 4) | (1u << 16))
+__device__ __forceinline__ void split_mma(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, bool accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 x, y;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "mov.b64 x, {%1, %5};\n\tmov.b64 y, {%2, %5};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], x, y, %3, p;\n\t}"
+      ::"r"(d), "r"(a), "r"(b), "r"(idesc), "r"((uint32_t)accumulate), "r"(32u | (1u << 14) | (4u << 29)) : "memory");
+}
+__device__ __forceinline__ void lds16(uint32_t a, uint32_t* x) {
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]) : "r"(a) : "memory");
+}
+__device__ __forceinline__ void sts16(uint32_t a, const uint32_t* x) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(x[0]), "r"(x[1]), "r"(x[2]), "r"(x[3]) : "memory");
+}
+__device__ __forceinline__ void ld8(uint32_t taddr, float2* v) {
+  uint32_t r[8];
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr));
+#pragma unroll
+  for (int i = 0; i < 4; ++i) v[i] = make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+}
+__device__ __forceinline__ void add8(float2* a, const float2* v) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 y, {%2, %3};\n\tadd.rn.f32x2 x, x, y;\n\t"
+        "mov.b64 {%0, %1}, x;\n\t}" : "+f"(a[i].x), "+f"(a[i].y) : "f"(v[i].x), "f"(v[i].y));
+}
+__device__ __forceinline__ void st8(uint32_t taddr, const float2* v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(__float_as_uint(v[0].x)),
+               "r"(__float_as_uint(v[0].y)), "r"(__float_as_uint(v[1].x)), "r"(__float_as_uint(v[1].y)),
+               "r"(__float_as_uint(v[2].x)), "r"(__float_as_uint(v[2].y)), "r"(__float_as_uint(v[3].x)),
+               "r"(__float_as_uint(v[3].y)) : "memory");
+}
+__device__ __forceinline__ void less(uint32_t& a, uint32_t& b, uint32_t pa, uint32_t pb) {      // (a, b) -= (pa, pb), exact
+  asm("{\n\t.reg .b64 x, p;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 p, {%2, %3};\n\t"
+      "fma.rn.f32x2 x, p, %4, x;\n\tmov.b64 {%0, %1}, x;\n\t}" : "+r"(a), "+r"(b) : "r"(pa), "r"(pb), "l"(0xbf800000bf800000ull));
+}
+// Two numbers (their bits) to two words of parts, the first in the lower half.  Rounded, so that the rest has either sign and
+// the three products left out cancel; what is left for l is at most eight bits.
+__device__ __forceinline__ void split2(uint32_t a, uint32_t b, uint32_t& h, uint32_t& m, uint32_t& l) {
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(h) : "f"(__uint_as_float(b)), "f"(__uint_as_float(a)));
+  less(a, b, h << 16, h & 0xffff0000u);
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(m) : "f"(__uint_as_float(b)), "f"(__uint_as_float(a)));
+  less(a, b, m << 16, m & 0xffff0000u);
+  l = __byte_perm(a, b, 0x7632);
 }
 
 // the product's last step: z (bias included), or with inv_tau > 0 a decay, sigmoid(z)^inv_tau
@@ -68,142 +110,328 @@ __device__ __forceinline__ float finish(float z, float inv_tau) {
   const float sp = -z > 20.f ? -z : log1pf(expf(-z));      // -log sigmoid(z)
   return expf(-sp * inv_tau);
 }
+// an output by plain multiply-adds, runs in ascending order: for sums that the split numbers cannot form
+__device__ __noinline__ float plain_dot(const float* __restrict__ a, const float* __restrict__ w, int K, int run) {
+  float tot = 0.f;
+  for (int k0 = 0; k0 < K; k0 += run) {
+    float s = 0.f;
+    for (int k = k0; k < min(K, k0 + run); ++k) s = fmaf(a[k], w[k], s);
+    tot = k0 ? tot + s : s;
+  }
+  return tot;
+}
+__device__ __forceinline__ bool is_finite(float z) { return (__float_as_uint(z) & 0x7f800000u) != 0x7f800000u; }
 
-// A tile of BM x BN outputs; a thread owns rows ty + NY i and columns tx + NX j.  SPLIT: the CTA of rank r in its
-// cluster of GROUPS computes run r, then every CTA adds up an eighth of the tile through distributed shared memory.
-template <int BM, int BN, int TM, int TN, bool VEC, bool SPLIT>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN), 4)
+// NT: the most rows of A that a tile can hold; `n` of them are this launch's (a multiple of 16).
+template <int NT> struct F32Shape {
+  static constexpr int SPLITTERS = NT >= 64 ? 12 : NT >= 32 ? 10 : 9;      // warps that split, ..
+  static constexpr int ADDERS = NT >= 64 ? 8 : 4;                   // that add up, and the one that issues the MMAs
+  static constexpr bool UNEQUAL = NT > 64;                          // registers by role (a warpgroup for the MMAs then)
+  static constexpr int WARPS = SPLITTERS + ADDERS;
+  static constexpr int THREADS = 32 * (WARPS + (UNEQUAL ? 4 : 1));
+  static constexpr int BLOCKS = NT / (2 * ADDERS);                  // blocks of 8 columns that a warp adds up
+  static constexpr int ROWS = 128 + NT;                             // of W, then of A
+  static constexpr int PASS = 8 * SPLITTERS;                        // rows that the splitting threads take at a time
+  static constexpr int PASSES = (ROWS + PASS - 1) / PASS;
+  static constexpr int LAST = ROWS - (PASSES - 1) * PASS;           // rows of the last pass
+  static constexpr int SLOTS = NT == 64 ? 3 : 2;     // stages of split rows
+  static constexpr int RAW = NT == 32 ? 2 : NT == 64 ? 4 : 3;          // stages of 32-bit rows in flight
+  static constexpr int RAW_STAGE = ROWS * 128;
+  static constexpr int SPLIT_STAGE = 3 * ROWS * 64;
+  static constexpr int BAR_OFF = RAW * RAW_STAGE + SLOTS * SPLIT_STAGE;
+  static constexpr int SMEM = BAR_OFF + 128 + 1024 /*alignment*/;
+  static constexpr int CTAS = NT <= 32 ? 2 : 1;                     // per processor
+  static constexpr int TMEM_COLS = NT <= 16 ? 128 : NT <= 32 ? 256 : 512;      // four times n of them used, or five times
+  static_assert(BAR_OFF >= 128 * NT * 4, "the partial sums take the tiles' place");
+  static_assert(CTAS * (SMEM + 1024) <= 233472, "what a CTA may have");
+};
+
+// CS: the CTAs of a cluster that share a tile, GROUPS / CS runs each; with several, each then adds up its part of the tile
+// through distributed shared memory.  VEC: both operands' rows can be copied 16 bytes at a time.
+template <int NT, bool VEC, int CS>
+__global__ void __launch_bounds__(F32Shape<NT>::THREADS, F32Shape<NT>::CTAS)
 gemm_f32_nt_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw,
                    const float* __restrict__ bias, float* __restrict__ C, int ldc, int M, int N, int K, int run,
-                   float inv_tau) {
-  constexpr int NX = BN / TN, NY = BM / TM, T = NX * NY;
-  constexpr int STAGE = (BM + BN) * KP;
-  extern __shared__ __align__(16) float smem[];
-  pdl_wait();
-  pdl_trigger();
-  const int tx = threadIdx.x % NX, ty = threadIdx.x / NX;
-  const int rank = SPLIT ? (int)(blockIdx.x % GROUPS) : 0;      // the cluster lies along x
-  const int m0 = blockIdx.y * BM, n0 = (SPLIT ? blockIdx.x / GROUPS : blockIdx.x) * BN;
-  const int kbegin = SPLIT ? min(K, rank * run) : 0, kend = SPLIT ? min(K, kbegin + run) : K;
+                   float inv_tau, int n) {
+  using S = F32Shape<NT>;
+  constexpr int BLOCKS = S::BLOCKS, RAW = S::RAW, SLOTS = S::SLOTS, PASSES = S::PASSES, STEP = S::ADDERS / 4;
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  unsigned char* split_base = base;              // [SLOTS][wh | wm | wl | ah | am | al], rows of 64 bytes
+  unsigned char* raw_base = base + SLOTS * S::SPLIT_STAGE;
+  uint64_t* full = reinterpret_cast<uint64_t*>(base + S::BAR_OFF);      // SLOTS: a stage is stored
+  uint64_t* done = full + SLOTS;                 // SLOTS: a stage is multiplied
+  uint64_t* lead_read = done + SLOTS;            // a stage's leading sums have been read
+  uint64_t* rest_read = lead_read + 1;           // a run's other sums have been read
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(rest_read + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = (int)(blockIdx.x % CS), share_k = run * (GROUPS / CS);      // the cluster lies along x
+  const int m0 = blockIdx.y * n, n0 = (blockIdx.x / CS) * 128;
+  const int kbegin = min(K, rank * share_k), kend = min(K, kbegin + share_k);
   const int tiles = (kend - kbegin + BK - 1) / BK, per_run = run / BK;
 
-  unsigned long long acc[TM][TN];
-  float tot[TM][TN];
-#pragma unroll
-  for (int i = 0; i < TM; ++i)
-#pragma unroll
-    for (int j = 0; j < TN; ++j) { acc[i][j] = 0ull; tot[i][j] = 0.f; }
+  // W's first stages on their way to the L2 while the kernel before this one ends: a hint, which reads nothing that it writes
+  if (warp < S::SPLITTERS && n <= 64) {
+    for (int x = threadIdx.x >> 2; x < 128 && n0 + x < N; x += S::PASS)
+      for (int k = kbegin + (threadIdx.x & 3) * 32; k < min(kend, kbegin + EARLY); k += 128)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(W + (size_t)(n0 + x) * ldw + k));
+  }
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < SLOTS; ++i) { at_bar_init(full + i, S::SPLITTERS); at_bar_init(done + i, 1); }
+    at_bar_init(lead_read, S::ADDERS);
+    at_bar_init(rest_read, S::ADDERS);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == S::WARPS) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(at_smem(tmem_slot)), "r"(S::TMEM_COLS));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;              // columns: n of a stage's leading sums, 2n of a run's others, n or 2n of runs
+  pdl_wait();
+  pdl_trigger();
 
-  // A thread copies the same four k of rows CR apart.  Inside the matrices that is an addition per copy: rows of A
-  // below the last one read the last one (their outputs are not stored), W's rows lie a fixed step apart.
-  constexpr int CR = T / (BK / 4), AR = BM > CR ? BM / CR : 1, WR = BN / CR;
-  static_assert(BN % CR == 0 && (BM % CR == 0 || BM < CR), "whole rounds of copies");
-  const int cr = threadIdx.x / (BK / 4), ck = threadIdx.x % (BK / 4) * 4;
-  const float* ap[AR];
+  bool ok = true;
+  // an adding warp's columns (rows of A): blocks first, first + STEP, ..
+  const int first = STEP == 2 ? (warp >> 2) & 1 : 0, blocks = n / 8;
+  float* part = reinterpret_cast<float*>(base);  // [n][128]: the sums, once nothing reads or writes the stages any more
+  if (warp >= S::WARPS) {
+    if (S::UNEQUAL) asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+    if (warp == S::WARPS && lane == 0) {
+      constexpr uint32_t kind = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 4) << 24);
+      const uint32_t one = kind | ((uint32_t)(n >> 3) << 17), two = kind | ((uint32_t)(n >> 2) << 17);
+      const uint32_t rest = tmem + n, part = (uint32_t)n * 4, lo = SPLIT_DESC_LO(at_smem(split_base));
+      int in_run = 0, s = 0;
+      uint32_t phase = 0, run_phase = 1;
+      for (int t = 0; t < tiles; ++t) {
+        if (!at_wait(full + s, phase)) { ok = false; break; }
+        if (in_run == 0 && t > 0 && !at_wait(rest_read, run_phase)) { ok = false; break; }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t w = lo + s * (S::SPLIT_STAGE >> 4), a = w + (3 * W_PART >> 4);
+        constexpr uint32_t wpart = W_PART >> 4;
 #pragma unroll
-  for (int i = 0; i < AR; ++i) ap[i] = A + (size_t)min(m0 + cr + CR * i, M - 1) * lda + kbegin + ck;
-  const float* wp = W + (size_t)min(n0 + cr, N - 1) * ldw + kbegin + ck;
-  const size_t wstep = (size_t)CR * ldw;
-  const bool inside = n0 + BN <= N;
-  auto stage = [&](int t) {
-    if (t < tiles) {
-      float* s = smem + (t % STAGES) * STAGE;
-      const int k0 = kbegin + t * BK;
-      if (VEC && inside && k0 + BK <= kend) {
-        float* d = s + cr * KP + ck;
-        if (BM >= CR || cr < BM) {
-#pragma unroll
-          for (int i = 0; i < AR; ++i) cp_async16(d + CR * i * KP, ap[i] + t * BK, 16);
+        for (int k = 0; k < BK / 16; ++k) {
+          split_mma(rest, w + 2 * k, a + part + 2 * k, two, in_run > 0 || k > 0);      // wh am | wh al
+          split_mma(rest, w + wpart + 2 * k, a + 2 * k, two, true);                    // wm ah | wm am
+          split_mma(rest + n, w + 2 * wpart + 2 * k, a + 2 * k, one, true);            // wl ah
         }
-        const float* w = wp + t * BK;
+        // The leading products last: meanwhile the sums of the stage before have been read
+        if (t > 0 && !at_wait(lead_read, (t - 1) & 1)) { ok = false; break; }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-        for (int i = 0; i < WR; ++i) cp_async16(d + (BM + CR * i) * KP, w + i * wstep, 16);
-      } else {
-        stage_rows<BM, T, VEC>(s, A, lda, m0, M, k0, kend);
-        stage_rows<BN, T, VEC>(s + BM * KP, W, ldw, n0, N, k0, kend);
+        for (int k = 0; k < BK / 16; ++k) split_mma(tmem, w + 2 * k, a + 2 * k, one, k > 0);
+        at_commit(done + s);
+        if (++in_run == per_run) { in_run = 0; run_phase ^= 1; }
+        if (++s == SLOTS) { s = 0; phase ^= 1; }
       }
+      if (!ok) atomicExch(&gemm_f32_stuck, 41);
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");       // an empty group past the end keeps the count
-  };
+  } else if (warp < S::SPLITTERS) {
+    if (S::UNEQUAL) asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+    // Thread q of a row's four takes the 16-byte pieces q and q + 4 of its 32 numbers (a warp's copy then reads whole
+    // sectors) and stores their parts as the row's 16-byte piece q: both operands' k are permuted the same way.
+    // Rows past A's end keep whatever is there, rows past W's end read its last one: their outputs are not stored.  (All
+    // sixteen rows of a tile reading one row of A cost a single row of 16384x2048 4 us: every CTA asks for the same lines.)
+    const int q = threadIdx.x & 3, row = threadIdx.x >> 2;
+    const float* src[PASSES];
+    bool mine[PASSES];
 #pragma unroll
-  for (int t = 0; t < STAGES - 1; ++t) stage(t);
-  int in_run = 0;
-  bool first = true;
+    for (int p = 0; p < PASSES; ++p) {
+      const int x = row + S::PASS * p;
+      mine[p] = x < 128 + min(n, M - m0);
+      src[p] = (x < 128 ? W + (size_t)min(n0 + x, N - 1) * ldw : A + (size_t)(mine[p] ? m0 + x - 128 : 0) * lda) + kbegin + q * 4;
+    }
+    const uint32_t raw = at_smem(raw_base) + threadIdx.x * 16;
+    constexpr int PIECES = S::PASS * 64, LAST_PIECES = S::LAST * 64;      // bytes of a pass's first pieces
+    int left = kend - kbegin - q * 4;              // k from this thread's first piece of the next stage to the end
+    uint32_t slot = raw;
+    auto fetch = [&]() {                           // the next stage into the next slot
+      if (VEC && left >= 20) {
+#pragma unroll
+        for (int p = 0; p < PASSES; ++p) {
+          if (S::PASS * (p + 1) > 128 && !mine[p]) continue;
+          cp_async16(slot + p * 2 * PIECES, src[p], 16);
+          cp_async16(slot + p * 2 * PIECES + (p < PASSES - 1 ? PIECES : LAST_PIECES), src[p] + 16, 16);
+        }
+      } else if (left > -q * 4) {
+#pragma unroll
+        for (int p = 0; p < PASSES; ++p) {
+          if (!mine[p]) continue;
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+#pragma unroll
+            for (int e = 0; e < 4; e += VEC ? 4 : 1) {
+              const bool in = h * 16 + e < left;
+              const float* from = in ? src[p] + h * 16 + e : A;
+              const uint32_t to = slot + p * 2 * PIECES + h * (p < PASSES - 1 ? PIECES : LAST_PIECES) + 4 * e;
+              if (VEC) cp_async16(to, from, in ? 16 : 0);
+              else cp_async4(to, from, in ? 4 : 0);
+            }
+          }
+        }
+      }
+      left -= BK;
+#pragma unroll
+      for (int p = 0; p < PASSES; ++p) src[p] += BK;
+      slot = slot == raw + (RAW - 1) * S::RAW_STAGE ? raw : slot + S::RAW_STAGE;
+      asm volatile("cp.async.commit_group;" ::: "memory");       // an empty group past the end keeps the count
+    };
 #pragma unroll 1
-  for (int t = 0; t < tiles; ++t) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
-    __syncthreads();                       // tile t is there for everybody; the buffer of tile t - 1 is free
-    stage(t + STAGES - 1);
-    const float* a_s = smem + (t % STAGES) * STAGE + ty * KP;
-    const float* w_s = smem + (t % STAGES) * STAGE + (BM + tx) * KP;
+    for (int t = 0; t < RAW; ++t) fetch();
+    const uint32_t to = at_smem(split_base) + ((q ^ ((row >> 1) & 3)) << 4);
+    int s = 0;
+    uint32_t phase = 1;
+#pragma unroll 1
+    for (int t = 0; t < tiles; ++t) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(RAW - 1) : "memory");
+      if (t >= SLOTS && !at_wait(done + s, phase)) ok = false;
+      if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+      uint32_t x[PASSES][8];
 #pragma unroll
-    for (int k = 0; k < BK; k += 4) {
-
-      ulonglong2 a[TM], w[TN];
-#pragma unroll
-      for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(a_s + i * NY * KP + k);
-#pragma unroll
-      for (int j = 0; j < TN; ++j) w[j] = *reinterpret_cast<const ulonglong2*>(w_s + j * NX * KP + k);
-#pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = fma2(a[i].x, w[j].x, acc[i][j]);
-#pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = fma2(a[i].y, w[j].y, acc[i][j]);
-    }
-    if (++in_run == per_run || t == tiles - 1) {
-#pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) {
-          tot[i][j] = first ? pair_sum(acc[i][j]) : tot[i][j] + pair_sum(acc[i][j]);
-          acc[i][j] = 0ull;
-        }
-      in_run = 0;
-      first = false;
-    }
-  }
-  if (!SPLIT) {
-#pragma unroll
-    for (int i = 0; i < TM; ++i) {
-      const int m = m0 + ty + NY * i;
-      if (m >= M) continue;
-#pragma unroll
-      for (int j = 0; j < TN; ++j) {
-        const int n = n0 + tx + NX * j;
-        if (n < N) C[(size_t)m * ldc + n] = finish(tot[i][j] + (bias ? bias[n] : 0.f), inv_tau);
+      for (int p = 0; p < PASSES; ++p) {
+        if (S::PASS * (p + 1) > 128 && !mine[p]) continue;
+        lds16(slot + p * 2 * PIECES, x[p]);
+        lds16(slot + p * 2 * PIECES + (p < PASSES - 1 ? PIECES : LAST_PIECES), x[p] + 4);
       }
+#pragma unroll
+      for (int p = 0; p < PASSES; ++p) {
+        if (S::PASS * (p + 1) > 128 && !mine[p]) continue;
+        uint32_t h[4], m[4], l[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) split2(x[p][2 * e], x[p][2 * e + 1], h[e], m[e], l[e]);
+        const int x = row + S::PASS * p;           // (PASS is a multiple of 8: the swizzle is the same in all passes)
+        const bool a = S::PASS * (p + 1) > 128 && x >= 128;
+        const uint32_t o = to + s * S::SPLIT_STAGE + x * 64 + (a ? 2 * W_PART : 0), part = a ? (uint32_t)n * 64 : W_PART;
+        sts16(o, h);
+        sts16(o + part, m);
+        sts16(o + 2 * part, l);
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) at_arrive(full + s);
+      fetch();                                     // into the pieces that this thread has just read
+      if (++s == SLOTS) { s = 0; phase ^= 1; }
     }
-    return;
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    if (!ok && lane == 0) atomicExch(&gemm_f32_stuck, 42);
+  } else {
+    if (S::UNEQUAL) asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
+    const uint32_t at = tmem + ((uint32_t)((warp & 3) * 32) << 16) + first * 8;     // its lanes of TMEM: rows of W
+    float2 acc[BLOCKS][4];                       // the run's sums, in the end all runs'
+#pragma unroll
+    for (int i = 0; i < BLOCKS; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[i][e] = make_float2(0.f, 0.f);
+    int in_run = 0, run_index = 0, s = 0;
+    uint32_t phase = 0;
+#pragma unroll 1
+    for (int t = 0; t < tiles; ++t) {
+      if (!at_wait(done + s, phase)) ok = false;
+      if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+      for (int i = 0; i < BLOCKS; i += 2) {
+        float2 v[2][4];
+        const bool one = first + STEP * i < blocks, two = i + 1 < BLOCKS && first + STEP * (i + 1) < blocks;
+        if (one) ld8(at + STEP * 8 * i, v[0]);
+        if (two) ld8(at + STEP * 8 * (i + 1), v[1]);
+        at_ld_wait();
+        if (one) add8(acc[i], v[0]);
+        if (two) add8(acc[i + 1 < BLOCKS ? i + 1 : i], v[1]);
+      }
+      const bool last = t == tiles - 1, close = ++in_run == per_run || last;
+      if (close) {                                 // the run's sum; the sums of the runs before wait in TMEM
+        const bool more = run_index % (GROUPS / 2) != 0;
+#pragma unroll
+        for (int i = 0; i < BLOCKS; ++i) {
+          if (first + STEP * i >= blocks) continue;
+          const uint32_t col = at + STEP * 8 * i;
+          float2 d[4], d2[4];
+          ld8(col + n, d);
+          ld8(col + 2 * n, d2);
+          at_ld_wait();
+          add8(d, d2);
+          add8(acc[i], d);
+          if (more) {
+            ld8(col + 3 * n, d);
+            at_ld_wait();
+            add8(acc[i], d);
+          }
+          if (CS == 1 && last && run_index >= GROUPS / 2) {
+            ld8(col + 4 * n, d);
+            at_ld_wait();
+            add8(acc[i], d);
+          }
+          if (!last) {
+            st8(col + (3 + (CS == 1 && run_index == GROUPS / 2 - 1)) * n, acc[i]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[i][e] = make_float2(0.f, 0.f);
+          }
+        }
+        ++run_index;
+        at_st_wait();
+        in_run = 0;
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) {
+        at_arrive(lead_read);
+        if (close) at_arrive(rest_read);
+      }
+      if (++s == SLOTS) { s = 0; phase ^= 1; }
+    }
+    if (!ok && lane == 0) atomicExch(&gemm_f32_stuck, 43);
+    // The sums go through shared memory (the last stage is multiplied: nothing reads or writes the stages any more) and are
+    // finished in a loop: 64 of them a thread in straight line took 9 us, most of it to fetch the instructions.
+    float* mine = part + first * 8 * 128 + (warp & 3) * 32 + lane;
+    const float spoilt = ok ? 0.f : __uint_as_float(0x7fc00000u);
+#pragma unroll
+    for (int i = 0; i < BLOCKS; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (first + STEP * i < blocks) {
+          mine[(STEP * 8 * i + 2 * e) * 128] = ok ? acc[i][e].x : spoilt;
+          mine[(STEP * 8 * i + 2 * e + 1) * 128] = ok ? acc[i][e].y : spoilt;
+        }
   }
-  __syncthreads();                         // the last tile has been read; no copy is in flight (only empty groups)
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == S::WARPS)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(S::TMEM_COLS));
+  if (CS > 1) asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  const int runs = (K + run - 1) / run, share = n * 128 / CS;
+  const uint32_t own = at_smem(part);
+  // (the warps that have the fewest registers stay out)
+  const int end = warp < S::WARPS ? (rank + 1) * share : 0;
+#pragma unroll 1
+  for (int e = rank * share + threadIdx.x; e < end; e += 32 * S::WARPS) {
+    const int m = m0 + e / 128, nn = n0 + e % 128;
+    if (m >= M || nn >= N) continue;
+    float z = part[e];
+    if (CS > 1) {
+      float v[CS];
 #pragma unroll
-  for (int i = 0; i < TM; ++i)
+      for (int g = 0; g < CS; ++g) {
+        uint32_t far;
+        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(far) : "r"(own + 4u * e), "r"(g));
+        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v[g]) : "r"(far));
+      }
+      float lo = v[0], hi = v[CS / 2];
 #pragma unroll
-    for (int j = 0; j < TN; ++j) smem[(ty + NY * i) * BN + tx + NX * j] = tot[i][j];
-  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-  const int runs = (K + run - 1) / run;
-  const unsigned mine = (unsigned)__cvta_generic_to_shared(smem);
-  for (int e = rank * (BM * BN / GROUPS) + threadIdx.x; e < (rank + 1) * (BM * BN / GROUPS); e += T) {
-    const int m = m0 + e / BN, n = n0 + e % BN;
-    if (m >= M || n >= N) continue;
-    float v[GROUPS];
-#pragma unroll
-    for (int g = 0; g < GROUPS; ++g) {
-      unsigned there;
-      asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(mine + 4u * e), "r"(g));
-      asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v[g]) : "r"(there));
+      for (int g = 1; g < CS / 2; ++g) {
+        if (g < runs) lo += v[g];
+        if (CS / 2 + g < runs) hi += v[CS / 2 + g];
+      }
+      z = runs > GROUPS / 2 ? lo + hi : lo;
     }
-    float sum = v[0];
-#pragma unroll
-    for (int g = 1; g < GROUPS; ++g)
-      if (g < runs) sum += v[g];
-    C[(size_t)m * ldc + n] = finish(sum + (bias ? bias[n] : 0.f), inv_tau);
+    if (!is_finite(z)) z = plain_dot(A + (size_t)m * lda, W + (size_t)nn * ldw, K, run);
+    C[(size_t)m * ldc + nn] = finish(z + (bias ? bias[nn] : 0.f), inv_tau);
   }
   // nobody leaves while its partial sums may still be read
-  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (CS > 1) asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 struct F32Problem {
@@ -211,25 +439,25 @@ struct F32Problem {
   float* C;
   int lda, ldw, ldc, M, N, K, run;
   float inv_tau;
+  int n;
   cudaStream_t stream;
 };
 
-template <int BM, int BN, int TM, int TN, bool VEC, bool SPLIT>
+template <int NT, bool VEC, int CS>
 static int launch_f32(const F32Problem& p) {
-  constexpr int smem = STAGES * (BM + BN) * KP * 4;
-  static_assert(smem >= BM * BN * 4 && (BM * BN) % GROUPS == 0, "the partial sums take the tiles' place");
-  auto kernel = gemm_f32_nt_kernel<BM, BN, TM, TN, VEC, SPLIT>;
+  constexpr int smem = F32Shape<NT>::SMEM;
+  auto kernel = gemm_f32_nt_kernel<NT, VEC, CS>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return AB_CUDA_ERR + (int)e;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((p.N + BN - 1) / BN * (SPLIT ? GROUPS : 1), (p.M + BM - 1) / BM);
-  cfg.blockDim = dim3((BM / TM) * (BN / TN));
+  cfg.gridDim = dim3((p.N + 127) / 128 * CS, (p.M + p.n - 1) / p.n);
+  cfg.blockDim = dim3(F32Shape<NT>::THREADS);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = p.stream;
   cudaLaunchAttribute attr[2];
-  if (SPLIT) {
+  if (CS > 1) {
     attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
-    attr[cfg.numAttrs].val.clusterDim.x = GROUPS;
+    attr[cfg.numAttrs].val.clusterDim.x = CS;
     attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
     ++cfg.numAttrs;
   }
@@ -239,14 +467,14 @@ static int launch_f32(const F32Problem& p) {
     ++cfg.numAttrs;
   }
   cfg.attrs = attr;
-  e = cudaLaunchKernelEx(&cfg, kernel, p.A, p.lda, p.W, p.ldw, p.bias, p.C, p.ldc, p.M, p.N, p.K, p.run, p.inv_tau);
+  e = cudaLaunchKernelEx(&cfg, kernel, p.A, p.lda, p.W, p.ldw, p.bias, p.C, p.ldc, p.M, p.N, p.K, p.run, p.inv_tau, p.n);
   return e == cudaSuccess ? AB_OK : AB_CUDA_ERR + (int)e;
 }
 
-template <int BM, int BN, int TM, int TN>
-static int launch_f32(const F32Problem& p, bool vec, bool split) {
-  if (vec) return split ? launch_f32<BM, BN, TM, TN, true, true>(p) : launch_f32<BM, BN, TM, TN, true, false>(p);
-  return split ? launch_f32<BM, BN, TM, TN, false, true>(p) : launch_f32<BM, BN, TM, TN, false, false>(p);
+template <int NT>
+static int launch_f32(const F32Problem& p, bool vec, int cs) {
+  if (vec) return cs == 1 ? launch_f32<NT, true, 1>(p) : cs == 2 ? launch_f32<NT, true, 2>(p) : launch_f32<NT, true, 8>(p);
+  return cs == 1 ? launch_f32<NT, false, 1>(p) : cs == 2 ? launch_f32<NT, false, 2>(p) : launch_f32<NT, false, 8>(p);
 }
 
 static int gemm_f32(const float* A, int lda, const float* W, int ldw, const float* bias, float* C, int ldc, int M, int N,
@@ -254,7 +482,7 @@ static int gemm_f32(const float* A, int lda, const float* W, int ldw, const floa
   if (M <= 0 || N <= 0) return AB_OK;
   if (K < 0) return AB_BAD_ARG;
   if ((M + 63) / 64 > 65535) return AB_BAD_ARG;
-  F32Problem p{A, W, bias, C, lda, ldw, ldc, M, N, K, 0, inv_tau, stream};
+  F32Problem p{A, W, bias, C, lda, ldw, ldc, M, N, K, 0, inv_tau, 0, stream};
   p.run = ((K + GROUPS - 1) / GROUPS + BK - 1) / BK * BK;
   if (p.run < SHORTEST) p.run = SHORTEST;
   // 16-byte copies where every row of both operands starts on a 16-byte boundary and ends on one
@@ -262,20 +490,30 @@ static int gemm_f32(const float* A, int lda, const float* W, int ldw, const floa
   int sms = 148, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  // Split a tile's runs over a cluster where there are few tiles per SM: an SM needs three or four CTAs to fill its
-  // pipes, and the last round is as long as a run.  us whole / split: 333 rows of 2048x2048 (1.2 tiles per SM) 122 / 87,
-  // 777 of 3072x2048 (4.1) 280 / 259, 2,048 of 2048x2048 (6.9) 391 / 425, 333 of 16384x2048 (9.5) 573 / 590.
-  auto split = [&](int bm, int bn) {
-    const long long tiles = (long long)((M + bm - 1) / bm) * ((N + bn - 1) / bn);
-    return K >= 512 && tiles < 6LL * sms;
-  };
-  // Few rows are bound by the weights' bytes and the chain of a run: as low a tile as holds them.
-  if (M <= 8) return launch_f32<8, 128, 8, 1>(p, vec, split(8, 128));
-  if (M <= 16 || (M <= 32 && N <= 8192)) return launch_f32<16, 128, 8, 2>(p, vec, split(16, 128));
-  // The tile that pads fewer rows; of equals the square one (2,048 rows: 4 % faster).
-  const long long low = (M + 31) / 32 * 32LL, square = (M + 63) / 64 * 64LL;
-  if (low < square * 0.97 && low / 32 <= 65535) return launch_f32<32, 128, 8, 4>(p, vec, split(32, 128));
-  return launch_f32<64, 64, 8, 4>(p, vec, split(64, 64));
+  // as few tiles of rows as 128 allow, then as low as they can be
+  // (where a tile is one short run and 64 rows leave processors idle, by 64: 200 rows of 2048x128 11.4 -> 8.7 us)
+  const int top = K <= SHORTEST && (long long)((N + 127) / 128) * ((M + 63) / 64) <= sms ? 64 : 128;
+  const int row_tiles = (M + top - 1) / top;
+  p.n = ((M + row_tiles - 1) / row_tiles + 15) / 16 * 16;
+  const long long tiles = (long long)((N + 127) / 128) * row_tiles;
+  const int resident = p.n <= 32 ? 2 * sms : sms;
+  // CTAs per tile: rounds of CTAs times what one takes, in stages of k (it starts and ends in about 8 of them; clusters leave a
+  // tenth of the processors unused).  us with 1 / 2 / 8: one row of 16384x2048 54 / 39 / 54, of 3072x2048 50 / 27 / 13; 200 rows of
+  // 3072x2048 44 / 44 / 59, of 2048x8192 133 / 133 / 112.
+  const long long runs = (K + p.run - 1) / p.run;
+  int cs = 1;
+  long long best = 0;
+  for (int c : {1, 2, 8}) {
+    if (c == 1 && p.n > 96 && runs > GROUPS / 2) continue;      // no room for the second sum of runs
+    if (c > runs && c > 1) continue;
+    const long long at_once = c == 1 ? resident : resident * 9 / 10;
+    const long long cost = (tiles * c + at_once - 1) / at_once * ((runs + c - 1) / c * (p.run / BK) + 8);
+    if (!best || cost < best) { best = cost; cs = c; }
+  }
+  if (p.n <= 16) return launch_f32<16>(p, vec, cs);
+  if (p.n <= 32) return launch_f32<32>(p, vec, cs);
+  if (p.n <= 64) return launch_f32<64>(p, vec, cs);
+  return launch_f32<128>(p, vec, cs);
 }
 
 AB_API int ab_gemm_f32_nt(const float* A, int lda, const float* W, int ldw, const float* bias, float* C, int ldc,
@@ -288,4 +526,11 @@ AB_API int ab_gemm_f32_decay(const float* A, int lda, const float* W, int ldw, c
                              int M, int N, int K, float tau, cudaStream_t stream) {
   if (!(tau > 0.f)) return AB_BAD_ARG;
   return gemm_f32(A, lda, W, ldw, bias, C, ldc, M, N, K, 1.0f / tau, stream);
+}
+
+AB_API int ab_gemm_f32_status() {
+  int v = 0, zero = 0;
+  if (cudaMemcpyFromSymbol(&v, gemm_f32_stuck, sizeof(int)) != cudaSuccess) return -1;
+  if (v) cudaMemcpyToSymbol(gemm_f32_stuck, &zero, sizeof(int));
+  return v;
 }

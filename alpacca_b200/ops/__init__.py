@@ -300,7 +300,8 @@ def attention_simt(qkv, out, k_pages, v_pages, block_table, tok_pos, tok_seq, n_
 
 
 def gemm_f32(a, w, out, bias=None, n_rows=None):
-    """out[M,N] = a[M,K] @ w[N,K]^T (+ bias) in true float32 (CUDA-core FMA, fixed k order)."""
+    """out[M,N] = a[M,K] @ w[N,K]^T (+ bias) with the precision of float32 sums in a fixed order: operands as exact sums of
+    three bfloat16 parts on the tensor cores."""
     _cuda(a, w, out, bias)
     _need(a.dtype == torch.float32 and w.dtype == torch.float32 and out.dtype == torch.float32,
           "gemm_f32 takes float32 tensors")
@@ -312,6 +313,7 @@ def gemm_f32(a, w, out, bias=None, n_rows=None):
           "gemm_f32: a [M,K], w [N,K], out [M,N], contiguous")
     if bias is not None:
         _need(bias.dtype == torch.float32 and bias.numel() == N and bias.is_contiguous(), "gemm_f32: bias f32 [N]")
+    _tc_unchecked["gemm_f32"] = True
     _check(_lib("gemm_f32").ab_gemm_f32_nt(_p(a), K, _p(w), K, _p(bias), _p(out), N, M, N, K, _stream()),
            "gemm_f32")
     return out
@@ -998,7 +1000,7 @@ TC_PAIR = True
 
 # kernels that wait on barriers with a limit, launched since the last check
 _tc_unchecked = {"gemm_tc": False, "attention_tc": False, "attention_pair_tc": False, "attention_latent_tc": False,
-                 "attention_stream": False}
+                 "attention_stream": False, "gemm_f32": False}
 
 
 def check_tc_status() -> None:
@@ -1009,7 +1011,7 @@ def check_tc_status() -> None:
     for name, read in (("gemm_tc", gemm_tc_status), ("attention_tc", attention_tc_status),
                        ("attention_pair_tc", attention_pair_tc_status),
                        ("attention_latent_tc", attention_latent_tc_status),
-                       ("attention_stream", attention_stream_status)):
+                       ("attention_stream", attention_stream_status), ("gemm_f32", gemm_f32_status)):
         if _tc_unchecked[name]:
             _tc_unchecked[name] = False
             code = read()
@@ -1036,6 +1038,11 @@ def attention_pair_tc_status() -> int:
 def attention_latent_tc_status() -> int:
     """0, or the code left by the tcgen05 kernel over a cached latent when it gave up a wait (synchronises)."""
     return _lib("attention_latent_tc").ab_attention_latent_tc_status()
+
+
+def gemm_f32_status() -> int:
+    """0, or the code left by a 32-bit product that gave up waiting on a barrier (synchronises)."""
+    return _lib("gemm_f32").ab_gemm_f32_status()
 
 
 def attention_stream_status() -> int:
@@ -2102,6 +2109,7 @@ def gla_decay(y, w2t, bias, tau, out, n_tokens):
           "gla_decay: out float32 [T, channels]")
     _need(tau > 0, "gla_decay: tau positive")
     w = w2t.t().contiguous()
+    _tc_unchecked["gemm_f32"] = True
     _check(_lib("gemm_f32").ab_gemm_f32_decay(_p(y), ldy, _p(w), rank, _p(bias), _p(out), channels, n_tokens, channels, rank,
                                               ctypes.c_float(tau), _stream()), "gla_decay")
     return out

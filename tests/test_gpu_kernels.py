@@ -679,6 +679,29 @@ def test_gemm_f32_ragged_k(M, N, K):
     assert ((out[:M].double() - want).abs() <= bound).all() and (out[M] == 7.0).all()
 
 
+@pytest.mark.parametrize("M,K", [(1, 96), (16, 2048), (40, 1100), (130, 513)])
+def test_gemm_f32_extreme_numbers(M, K):
+    """Numbers that no bfloat16 holds (above its largest), infinities and NaNs go where plain multiply-adds take them; numbers of
+    very unlike sizes, and of one sign, keep the bound of the tiles' test."""
+    from alpacca_b200 import ops
+    N = 150
+    a, w = rnd(M, K, seed=1), rnd(N, K, seed=2).abs()
+    a *= torch.exp2(torch.randint(-30, 30, (M, K), generator=torch.Generator().manual_seed(3)).float()).cuda()
+    a[:, 5], w[3, 7], w[4, 7] = 1.0, float("inf"), float("nan")
+    a[0, 9], w[:, 9] = 3.4e38, 1e-3
+    if M > 1:
+        a[M // 2, 11] = float("-inf")
+    out = torch.empty(M, N, device="cuda")
+    ops.gemm_f32(a, w, out)
+    want = a.double() @ w.double().T
+    assert torch.equal(out.isnan(), want.isnan()) and torch.equal(out.isposinf(), want.isposinf())
+    assert torch.equal(out.isneginf(), want.isneginf())
+    at = want.isfinite()
+    bound = 2.0 ** -22 * a.double().nan_to_num(0, 0, 0).norm(dim=1)[:, None] * w.double().nan_to_num(0, 0, 0).norm(dim=1)[None]
+    assert ((out.double() - want).abs() <= bound)[at].all() and at.any()
+    assert ops.gemm_f32_status() == 0
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("page", [1, 5, 8, 12, 20])
 @pytest.mark.parametrize("window", [0, 11])
