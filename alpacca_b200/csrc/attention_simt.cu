@@ -14,6 +14,14 @@
 // dependent shuffles, two exponentials and a load that nothing overlaps; eight at
 // a time are eight loads in flight, nine shuffles for their sums and one rescaling.
 // 333 tokens, 32 heads of 64 on 8, float32: 281 -> 169 us.
+//
+// Query heads that come in fours per KV head (attention_rows_kernel): a block takes four heads of eight tokens, a token per warp,
+// and brings 32 keys and values at a time to shared memory, by cp.async, the next 32 under the work on these.  For the scores
+// a lane has a key and forms its four products with the heads; the softmax is that of four runs of eight lanes; for the
+// values a lane has its dimensions.  Every sum is formed in the order of the kernel above, operation by operation, so a row's
+// bits do not depend on which of the two ran.  Bound by instructions (about nine per head and key and 32 lanes).  us one
+// warp per row / this: 333 tokens, 32 heads of 64 on 8, 156 / 53; of 128 212 / 101; 2,000 tokens 3,820 / 1,100; one token each
+// of 8 sequences of 2,000 keys (a block per token then) 597 / 170; of one key 3.2 / 4.5.
 #include "common.cuh"
 
 #define KEYS 8      // keys that a warp takes at a time; the exchanges below are written for 8
@@ -114,6 +122,222 @@ __global__ void attention_simt_kernel(const T* __restrict__ q, int q_stride, T* 
   }
 }
 
+// float32, D = 32 DPL, pages of a multiple of KEYS keys; see the head of the file.
+#define ROWS 4             // heads of a warp
+#define ROW_WARPS 8        // tokens of a block
+#define STEP 32            // keys at a time
+template <int DPL> struct RowsShape {
+  static constexpr int D = 32 * DPL;
+  static constexpr int KP = D + 4;                                   // a lane per key reads 16 bytes of its row: no bank twice
+  static constexpr int TILE = STEP * (KP + D);                       // floats of a step's keys and values
+  static constexpr int Q = 2 * TILE, P = Q + ROW_WARPS * ROWS * D, SMEM = (P + ROW_WARPS * ROWS * STEP) * 4;
+};
+
+template <int DPL>
+__global__ void __launch_bounds__(ROW_WARPS * 32)
+attention_rows_kernel(const float* __restrict__ q, int q_stride, float* __restrict__ out, const float* __restrict__ k_pages,
+                      const float* __restrict__ v_pages, const int* __restrict__ block_table, int table_width,
+                      const int* __restrict__ tok_pos, const int* __restrict__ tok_seq, const int* __restrict__ cu_q, int n_seqs,
+                      int n_tokens, int H, int K, int page_size, float scale, int window) {
+  using S = RowsShape<DPL>;
+  constexpr int D = S::D, T = ROW_WARPS * 32;
+  extern __shared__ __align__(16) float sm[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int h = blockIdx.y * ROWS, kh = h / (H / K);
+  // this block's tokens: one, or the next of its sequence's runs of ROW_WARPS (the last ones, which see most keys, first)
+  int t0 = blockIdx.x, t_end = t0 + 1;
+  if (cu_q) {
+    int tile = gridDim.x - 1 - blockIdx.x;
+    t_end = t0 = 0;
+    for (int i = 0; i < n_seqs; ++i) {
+      const int begin = cu_q[i], end = min(cu_q[i + 1], n_tokens), tiles = (end - begin + ROW_WARPS - 1) / ROW_WARPS;
+      if (tile < tiles) {
+        t0 = begin + tile * ROW_WARPS;
+        t_end = min(end, t0 + ROW_WARPS);
+        break;
+      }
+      tile -= max(tiles, 0);
+    }
+  }
+  if (t0 >= t_end) return;                         // more blocks than runs
+  const int b = tok_seq[t0];
+  if (b < 0) return;                               // rows without a sequence
+  const int t = t0 + warp;
+  const bool mine = t < t_end;
+  const int pos = mine ? tok_pos[t] : -1;
+  const int lo = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
+  float* q_s = sm + S::Q + warp * ROWS * D;
+  float* p_s = sm + S::P + warp * ROWS * STEP;
+  if (mine) {
+#pragma unroll
+    for (int i = 0; i < ROWS * DPL; ++i) q_s[lane + 32 * i] = q[(size_t)t * q_stride + (size_t)h * D + lane + 32 * i];
+  }
+  __syncwarp();
+  float acc[ROWS][DPL], m[ROWS], l[ROWS];
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) {
+    m[r] = -INFINITY;
+    l[r] = 0.f;
+#pragma unroll
+    for (int j = 0; j < DPL; ++j) acc[r][j] = 0.f;
+  }
+  int from = 0x7fffffff, to = -1;                  // what the block's tokens see
+  for (int i = t0; i < t_end; ++i) {
+    const int p = tok_pos[i];
+    to = max(to, p);
+    from = min(from, (window > 0 && p - window + 1 > 0) ? p - window + 1 : 0);
+  }
+  from -= from % KEYS;
+  const int* bt = block_table + (size_t)b * table_width;
+  auto stage = [&](int s0, int buf) {
+    if (s0 <= to) {
+      float* k_t = sm + buf * S::TILE;
+      for (int i = threadIdx.x; i < STEP * (D / 4); i += T) {
+        const int row = i / (D / 4), c = i % (D / 4) * 4;
+        const size_t at = key_place(bt, min(s0 + row, to), K, kh, page_size, D) + c;      // (past the end: no row uses it)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(k_t + row * S::KP + c)), "l"(k_pages + at));
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(k_t + STEP * S::KP + row * D + c)), "l"(v_pages + at));
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  stage(from, 0);
+  int buf = 0;
+  for (int s0 = from; s0 <= to; s0 += STEP, buf ^= 1) {
+    stage(s0 + STEP, buf ^ 1);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();
+    if (mine && s0 <= pos && s0 + STEP > lo) {
+      const float *k_row = sm + buf * S::TILE + lane * S::KP, *v_t = sm + buf * S::TILE + STEP * S::KP;
+      // the products of dimensions d and d + 32 (.. + 96) first, then a tree over d: 16 apart, 8, 4, 2, 1
+      auto part = [&](int a, float4* x) {      // d = 4 a .. 4 a + 3 of the four heads
+        float4 kk[DPL];
+#pragma unroll
+        for (int j = 0; j < DPL; ++j) kk[j] = *reinterpret_cast<const float4*>(k_row + 32 * j + 4 * a);
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+          x[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+          for (int j = 0; j < DPL; ++j) {
+            const float4 qq = *reinterpret_cast<const float4*>(q_s + r * D + 32 * j + 4 * a);
+            x[r].x = fmaf(qq.x, kk[j].x, x[r].x);
+            x[r].y = fmaf(qq.y, kk[j].y, x[r].y);
+            x[r].z = fmaf(qq.z, kk[j].z, x[r].z);
+            x[r].w = fmaf(qq.w, kk[j].w, x[r].w);
+          }
+        }
+      };
+      auto add = [](float4* x, const float4* y) {
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r)
+          x[r] = make_float4(__fadd_rn(x[r].x, y[r].x), __fadd_rn(x[r].y, y[r].y), __fadd_rn(x[r].z, y[r].z), __fadd_rn(x[r].w, y[r].w));
+      };
+      auto quarter = [&](int a, float4* x) {   // a, a + 4, a + 2, a + 6
+        float4 y[ROWS], z[ROWS];
+        part(a, x);
+        part(a + 4, y);
+        add(x, y);
+        part(a + 2, y);
+        part(a + 6, z);
+        add(y, z);
+        add(x, y);
+      };
+      float4 even[ROWS], odd[ROWS];
+      quarter(0, even);
+      quarter(1, odd);
+      add(even, odd);
+      // four runs of eight keys: a run's lanes have its scores, and every lane follows the runs before its own
+      const int key = s0 + lane, run = lane >> 3;
+      float corr[ROWS];
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) {
+        const float dot = __fadd_rn(__fadd_rn(even[r].x, even[r].z), __fadd_rn(even[r].y, even[r].w));
+        const float score = key < lo || key > pos ? -INFINITY : __fmul_rn(dot, scale);
+        float top = score;
+#pragma unroll
+        for (int o = 1; o < KEYS; o <<= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+        float before = m[r], after = m[r];       // the maximum before and after this lane's run
+#pragma unroll
+        for (int g = 0; g < STEP / KEYS; ++g) {
+          const float run_top = __shfl_sync(0xffffffffu, top, g * KEYS);
+          if (g < run) before = fmaxf(before, run_top);
+          if (g <= run) after = fmaxf(after, run_top);
+          m[r] = fmaxf(m[r], run_top);
+        }
+        // a run without a visible key changes nothing (before the first one all maxima are -inf)
+        corr[r] = after == before ? 1.0f : expf(before - after);
+        const float p = score == -INFINITY ? 0.f : expf(score - after);
+        float sum = p;
+#pragma unroll
+        for (int o = 1; o < KEYS; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+#pragma unroll
+        for (int g = 0; g < STEP / KEYS; ++g)
+          l[r] = fmaf(l[r], __shfl_sync(0xffffffffu, corr[r], g * KEYS), __shfl_sync(0xffffffffu, sum, g * KEYS));
+        p_s[r * STEP + lane] = p;
+      }
+      __syncwarp();
+#pragma unroll
+      for (int g = 0; g < STEP / KEYS; ++g) {
+        const int g0 = s0 + g * KEYS;
+        if (g0 > pos || g0 + KEYS <= lo) continue;             // the same for the whole warp
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+          const float c = __shfl_sync(0xffffffffu, corr[r], g * KEYS);
+#pragma unroll
+          for (int j = 0; j < DPL; ++j) acc[r][j] *= c;
+        }
+        const bool whole = g0 >= lo && g0 + KEYS - 1 <= pos;
+#pragma unroll
+        for (int i0 = 0; i0 < KEYS; i0 += 4) {
+          float4 pr[ROWS];
+#pragma unroll
+          for (int r = 0; r < ROWS; ++r) pr[r] = *reinterpret_cast<const float4*>(p_s + r * STEP + g * KEYS + i0);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int s = g0 + i0 + i;
+            if (!whole && (s < lo || s > pos)) continue;
+            const float* v_row = v_t + (g * KEYS + i0 + i) * D + DPL * lane;
+            float v[DPL];
+            if constexpr (DPL == 2) *reinterpret_cast<float2*>(v) = *reinterpret_cast<const float2*>(v_row);
+            else *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(v_row);
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r) {
+              const float p = i == 0 ? pr[r].x : i == 1 ? pr[r].y : i == 2 ? pr[r].z : pr[r].w;
+#pragma unroll
+              for (int j = 0; j < DPL; ++j) acc[r][j] = fmaf(p, v[j], acc[r][j]);
+            }
+          }
+        }
+      }
+    }
+    __syncthreads();                             // the buffer may be filled again
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  if (!mine) return;
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) {
+    const float inv = 1.0f / l[r];
+    float* o = out + ((size_t)t * H + h + r) * D + DPL * lane;
+#pragma unroll
+    for (int j = 0; j < DPL; ++j) o[j] = acc[r][j] * inv;
+  }
+}
+
+template <int DPL>
+static int launch_rows(const float* q, int q_stride, float* out, const float* k_pages, const float* v_pages, const int* block_table,
+                       int table_width, const int* tok_pos, const int* tok_seq, const int* cu_q, int n_seqs, int n_tokens, int H,
+                       int K, int page_size, float scale, int window, cudaStream_t stream) {
+  constexpr int smem = RowsShape<DPL>::SMEM;
+  const cudaError_t e = cudaFuncSetAttribute(attention_rows_kernel<DPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return AB_CUDA_ERR + (int)e;
+  // (a sequence's last run may be short: at most n_seqs more than the tokens fill)
+  const dim3 grid((unsigned)(cu_q ? (n_tokens + ROW_WARPS - 1) / ROW_WARPS + n_seqs : n_tokens), (unsigned)(H / ROWS));
+  attention_rows_kernel<DPL><<<grid, ROW_WARPS * 32, smem, stream>>>(q, q_stride, out, k_pages, v_pages, block_table, table_width,
+                                                                      tok_pos, tok_seq, cu_q, n_seqs, n_tokens, H, K, page_size,
+                                                                      scale, window);
+  return ab_launch_status();
+}
+
 template <typename T>
 static int launch(const void* q, int q_stride, void* out, const void* k_pages, const void* v_pages,
                   const int* block_table, int table_width, const int* tok_pos, const int* tok_seq, int n_tokens,
@@ -134,12 +358,20 @@ static int launch(const void* q, int q_stride, void* out, const void* k_pages, c
   return ab_launch_status();
 }
 
-AB_API int ab_attention_simt(const void* q, int q_stride, void* out, int dtype, const void* k_pages,
-                             const void* v_pages, const int* block_table, int table_width, const int* tok_pos,
-                             const int* tok_seq, int n_tokens, int H, int K, int D, int page_size, float scale,
-                             int window, cudaStream_t stream) {
+// cu_q (int [n_seqs + 1], or null): where the sequences' tokens begin, in prompts.  `single`: one token per sequence.  With one of
+// the two, the kernel of four heads is taken where it can be; the results are the same.
+AB_API int ab_attention_simt_rows(const void* q, int q_stride, void* out, int dtype, const void* k_pages,
+                                  const void* v_pages, const int* block_table, int table_width, const int* tok_pos,
+                                  const int* tok_seq, const int* cu_q, int n_seqs, int single, int n_tokens, int H, int K, int D,
+                                  int page_size, float scale, int window, cudaStream_t stream) {
   if (n_tokens <= 0) return AB_OK;
   if (D <= 0 || D > 256 || H <= 0 || K <= 0 || H % K || page_size <= 0) return AB_BAD_ARG;
+  if ((cu_q || single) && dtype == AB_F32 && (D == 64 || D == 128) && H / K % ROWS == 0 && H / ROWS <= 65535 && page_size % KEYS == 0 &&
+      (((uintptr_t)k_pages | (uintptr_t)v_pages) & 15) == 0) {
+    return (D == 64 ? launch_rows<2> : launch_rows<4>)((const float*)q, q_stride, (float*)out, (const float*)k_pages,
+                                                       (const float*)v_pages, block_table, table_width, tok_pos, tok_seq,
+                                                       single ? nullptr : cu_q, n_seqs, n_tokens, H, K, page_size, scale, window, stream);
+  }
   if (dtype == AB_F32)
     return launch<float>(q, q_stride, out, k_pages, v_pages, block_table, table_width, tok_pos, tok_seq,
                          n_tokens, H, K, D, page_size, scale, window, stream);
@@ -147,4 +379,12 @@ AB_API int ab_attention_simt(const void* q, int q_stride, void* out, int dtype, 
     return launch<bf16>(q, q_stride, out, k_pages, v_pages, block_table, table_width, tok_pos, tok_seq,
                         n_tokens, H, K, D, page_size, scale, window, stream);
   return AB_BAD_ARG;
+}
+
+AB_API int ab_attention_simt(const void* q, int q_stride, void* out, int dtype, const void* k_pages,
+                             const void* v_pages, const int* block_table, int table_width, const int* tok_pos,
+                             const int* tok_seq, int n_tokens, int H, int K, int D, int page_size, float scale,
+                             int window, cudaStream_t stream) {
+  return ab_attention_simt_rows(q, q_stride, out, dtype, k_pages, v_pages, block_table, table_width, tok_pos, tok_seq, nullptr, 0,
+                                0, n_tokens, H, K, D, page_size, scale, window, stream);
 }

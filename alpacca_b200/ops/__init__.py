@@ -277,12 +277,16 @@ def swiglu(gu, out, n_rows=None):
 
 
 def attention_simt(qkv, out, k_pages, v_pages, block_table, tok_pos, tok_seq, n_tokens, H, K, D, scale,
-                   window=0):
+                   window=0, cu_q=None, single=False):
     """Attention of every token over its sequence's cached keys, 32-bit arithmetic.
 
-    qkv [T,(H+2K)D] (the q part is read), out [T,H*D].
+    qkv [T,(H+2K)D] (the q part is read), out [T,H*D].  `cu_q` (int32 [B+1], where the sequences' tokens begin) in prompts, or
+    `single` where every sequence has one token: lets eight tokens, or the heads of one, share their keys; the same bits.
     """
-    _cuda(qkv, out, k_pages, v_pages, block_table, tok_pos, tok_seq)
+    _cuda(qkv, out, k_pages, v_pages, block_table, tok_pos, tok_seq, cu_q)
+    n_seqs = 0 if cu_q is None else cu_q.numel() - 1
+    if cu_q is not None:
+        _i32(cu_q, n_seqs + 1, "cu_q")
     _need(qkv.is_contiguous() and out.is_contiguous() and out.dtype == qkv.dtype and k_pages.dtype == qkv.dtype,
           "attention: q, out and cache must share one dtype and be contiguous")
     _need(out.numel() >= n_tokens * H * D, "attention: out too small")
@@ -292,10 +296,10 @@ def attention_simt(qkv, out, k_pages, v_pages, block_table, tok_pos, tok_seq, n_
     page_size = k_pages.shape[2]
     _need(tuple(k_pages.shape[1:]) == (K, page_size, D) and k_pages.shape == v_pages.shape
           and k_pages.is_contiguous() and v_pages.is_contiguous(), "attention: cache pages [n_pages,K,page,D]")
-    _check(_lib("attention_simt").ab_attention_simt(
+    _check(_lib("attention_simt").ab_attention_simt_rows(
         _p(qkv), qkv.shape[-1], _p(out), _dt(qkv), _p(k_pages), _p(v_pages), _p(block_table),
-        block_table.shape[1], _p(tok_pos), _p(tok_seq), n_tokens, H, K, D, page_size, ctypes.c_float(scale),
-        int(window or 0), _stream()), "attention_simt")
+        block_table.shape[1], _p(tok_pos), _p(tok_seq), _p(cu_q), n_seqs, 1 if single else 0, n_tokens, H, K, D, page_size,
+        ctypes.c_float(scale), int(window or 0), _stream()), "attention_simt")
     return out
 
 
@@ -764,8 +768,9 @@ def attention(qkv, out, cache, ctx, H, K, D, scale, window=0):
     else (the 32-bit path, other head sizes up to 256): the 32-bit kernel."""
     if qkv.dtype == torch.bfloat16 and D % 16 == 0 and D <= 256 and H // K <= 64:
         return attention_mma(qkv, out, cache, ctx, H, K, D, scale, window)
+    single = ctx.is_decode
     return attention_simt(qkv, out, cache.k, cache.v, cache.block_table, ctx.tok_pos, ctx.tok_seq,
-                          ctx.n_tokens, H, K, D, scale, window)
+                          ctx.n_tokens, H, K, D, scale, window, cu_q=None if single else ctx.cu_q[:ctx.n_seqs + 1], single=single)
 
 
 FUSE_ROPE_DECODE = True          # decode steps: rotation and append inside the attention kernel

@@ -728,3 +728,28 @@ def test_attention_simt_any_page_size(dtype, page, window):
         want = ref_attention(q[at:at + n], ks[b].double().cpu(), vs[b].double().cpu(), pos[at:at + n].cpu(), D ** -0.5, window)
         close(out[at:at + n].view(n, H, D), want, dtype, f"sequence {b}")
         at += n
+
+
+@pytest.mark.parametrize("H,K,D", [(4, 1, 64), (16, 2, 128)])
+@pytest.mark.parametrize("window", [0, 11, 70])
+@pytest.mark.parametrize("lengths,q_lens", [([37, 3, 130], [9, 3, 1]), ([200], [200]), ([33, 64, 1, 7], [33, 8, 1, 7]), ([65, 1, 32], [1, 1, 1])])
+def test_attention_32bit_of_four_heads_has_the_same_bits(H, K, D, window, lengths, q_lens):
+    """Eight tokens, or the heads of one, that share their keys against a warp per row: every sum is in the same order.  Rows without
+    a sequence stay as they are, and values that are not numbers stay with the rows that see them."""
+    from alpacca_b200 import ops
+    table, kp, vp = make_paged(lengths, sum(-(-n // 64) for n in lengths) + 2, K, D, torch.float32, seed=5)
+    kp.copy_(rnd(*kp.shape, seed=6))
+    vp.copy_(rnd(*vp.shape, seed=7))
+    vp[table[0, (lengths[0] - 1) // 64].item(), :, (lengths[0] - 1) % 64] = float("nan")      # the first sequence's last key
+    T = sum(q_lens)
+    qkv = 3 * rnd(T + 1, (H + 2 * K) * D, seed=8)
+    pos = torch.cat([torch.arange(n - q, n) for n, q in zip(lengths, q_lens)] + [torch.zeros(1)]).to(torch.int32).cuda()
+    seq = torch.cat([torch.full((q,), b) for b, q in enumerate(q_lens)] + [torch.full((1,), -1)]).to(torch.int32).cuda()
+    cu_q = torch.tensor([sum(q_lens[:b]) for b in range(len(q_lens) + 1)], dtype=torch.int32).cuda()
+    want, got, one = (torch.full((T + 1, H * D), 7.0, device="cuda") for _ in range(3))
+    ops.attention_simt(qkv, want, kp, vp, table, pos, seq, T + 1, H, K, D, D ** -0.5, window)
+    ops.attention_simt(qkv, got, kp, vp, table, pos, seq, T + 1, H, K, D, D ** -0.5, window, cu_q=cu_q)
+    ops.attention_simt(qkv, one, kp, vp, table, pos, seq, T + 1, H, K, D, D ** -0.5, window, single=True)
+    assert want[:T].isnan().any() and not want[:T].isnan().all()
+    for x in (got, one):
+        assert torch.equal(x.view(torch.int32), want.view(torch.int32)) or torch.equal(x.nan_to_num(9.0), want.nan_to_num(9.0))
