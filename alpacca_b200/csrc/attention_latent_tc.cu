@@ -51,15 +51,16 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
   uint64_t* k_empty = k_full + STAGES;           // STAGES
   uint64_t* s_full = k_empty + STAGES;           // 2
   uint64_t* p_full = s_full + 2;                 // 2
-  uint64_t* o_done = p_full + 2;                 // 1: completes once per product O += P_j V_j
+  // 2, for even and odd j: completes once per product O += P_j V_j (a warp that waits for product j may come when product
+  // j - 1 is not done yet, which one barrier could not tell from product j)
+  uint64_t* o_done = p_full + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     at_bar_init(q_full, 1);
     for (int s = 0; s < STAGES; ++s) { at_bar_init(k_full + s, 1); at_bar_init(k_empty + s, 1); }
-    for (int i = 0; i < 2; ++i) { at_bar_init(s_full + i, 1); at_bar_init(p_full + i, 128); }
-    at_bar_init(o_done, 1);
+    for (int i = 0; i < 2; ++i) { at_bar_init(s_full + i, 1); at_bar_init(p_full + i, 128); at_bar_init(o_done + i, 1); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -137,7 +138,7 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
         for (int k = 0; k < LT_KEYS / 16; ++k)     // 16 keys per MMA: 8 columns of P, 2 groups of 8 rows of the tile
           at_mma_ts(tmem + o_col, tmem + (j & 1) * 128 + k * 8, at_desc_mn(v_addr + k * 2048, Sh::PANEL), idesc_o,
                     (j > 0 || k > 0) ? 1u : 0u);
-        at_commit(o_done);
+        at_commit(o_done + (j & 1));
         at_commit(k_empty + s);
       }
     }
@@ -205,7 +206,7 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
       l_run += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
       if (j > 0 && __any_sync(0xffffffffu, move)) {
         // rescale this warp's rows of O in TMEM, after the product before this tile has landed there
-        if (!at_wait(o_done, (j - 1) & 1)) { atomicExch(status, 25); ok = false; }
+        if (!at_wait(o_done + ((j - 1) & 1), ((j - 1) >> 1) & 1)) { atomicExch(status, 25); ok = false; }
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -223,7 +224,7 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
       at_arrive(p_full + (j & 1));
     }
     if (ok) {
-      if (!at_wait(o_done, (n_tiles - 1) & 1)) { atomicExch(status, 27); ok = false; }
+      if (!at_wait(o_done + ((n_tiles - 1) & 1), ((n_tiles - 1) >> 1) & 1)) { atomicExch(status, 27); ok = false; }
       ok = __all_sync(0xffffffffu, ok);
     }
     if (ok) {

@@ -98,7 +98,10 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   uint64_t* kv_empty = kv_full + AT_STAGES;      // STAGES
   uint64_t* s_full = kv_empty + AT_STAGES;       // 2
   uint64_t* p_full = s_full + 2;                 // 2
-  uint64_t* o_done = p_full + 2;                 // 1: completes once per product O += P_j V_j
+  // 2, for even and odd j: completes once per product O += P_j V_j.  A softmax warp may be done with tile j while another
+  // is still in tile j - 1: product j - 1 is then not even issued.  With one barrier the first one's wait for product j
+  // would take the phase of product j - 2 for its own and let it read O without the last two products
+  uint64_t* o_done = p_full + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -116,8 +119,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   if (threadIdx.x == 0) {
     at_bar_init(q_full, 1);
     for (int s = 0; s < AT_STAGES; ++s) { at_bar_init(kv_full + s, 1); at_bar_init(kv_empty + s, 1); }
-    for (int i = 0; i < 2; ++i) { at_bar_init(s_full + i, 1); at_bar_init(p_full + i, 128); }
-    at_bar_init(o_done, 1);
+    for (int i = 0; i < 2; ++i) { at_bar_init(s_full + i, 1); at_bar_init(p_full + i, 128); at_bar_init(o_done + i, 1); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -193,7 +195,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         for (int k = 0; k < AT_KEYS / 16; ++k)     // 16 keys per MMA: 8 columns of P, 2 groups of 8 V rows
           at_mma_ts(tmem + Sh::O_COL, tmem + Sh::p_col(j) + k * 8, at_desc_mn(v_addr + k * 2048, Sm::KV_PANEL), idesc_t,
                     (j > 0 || k > 0) ? 1u : 0u);
-        at_commit(o_done);
+        at_commit(o_done + (j & 1));
         at_commit(kv_empty + s);                   // K and V of this stage are read when these MMAs are done
       }
     }
@@ -304,7 +306,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       }
       if (j > 0 && __any_sync(0xffffffffu, move)) {
         // rescale this warp's rows of O in TMEM, after the product before this tile has landed there
-        if (!at_wait(o_done, (j - 1) & 1)) { atomicExch(status, 15); ok = false; }
+        if (!at_wait(o_done + ((j - 1) & 1), ((j - 1) >> 1) & 1)) { atomicExch(status, 15); ok = false; }
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) { if (DIST) continue; else break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -343,7 +345,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       at_arrive(p_full + (j & 1));
     }
     if (ok && n_tiles > 0) {
-      if (!at_wait(o_done, (n_tiles - 1) & 1)) { atomicExch(status, 17); ok = false; }
+      if (!at_wait(o_done + ((n_tiles - 1) & 1), ((n_tiles - 1) >> 1) & 1)) { atomicExch(status, 17); ok = false; }
       ok = __all_sync(0xffffffffu, ok);
     }
     if (ok) {

@@ -753,3 +753,48 @@ def test_attention_32bit_of_four_heads_has_the_same_bits(H, K, D, window, length
     assert want[:T].isnan().any() and not want[:T].isnan().all()
     for x in (got, one):
         assert torch.equal(x.view(torch.int32), want.view(torch.int32)) or torch.equal(x.nan_to_num(9.0), want.nan_to_num(9.0))
+
+
+@pytest.mark.parametrize("form,H,K,D", [("plain", 32, 8, 64), ("plain", 4, 4, 64), ("plain", 8, 2, 128), ("latent", 16, 1, 256),
+                                        ("latent", 4, 1, 64)])
+def test_prompt_attention_waits_for_its_last_products(form, H, K, D):
+    """A prompt of many tiles on top of a held one, again and again: the same bits every time, and every row right.  A warp that
+    reads its rows before the last products have landed leaves out up to 128 of their keys, more than an eighth of a row's norm.
+    Bound: weights and outputs are rounded to 8 bits, 2^-9 each; random rows add up to about three times that, times 2.5."""
+    from alpacca_b200 import ops
+    from alpacca_b200.cache import KVLayerView
+    from types import SimpleNamespace
+    lengths, q_lens = [2200, 1500], [1490, 1500]
+    table, kp, vp = make_paged(lengths, 62, K, D, torch.bfloat16, seed=H)
+    kp.copy_(rnd(*kp.shape, seed=1))
+    vp.copy_(rnd(*vp.shape, seed=2))
+    T = sum(q_lens)
+    cu = torch.tensor([0, q_lens[0], T], dtype=torch.int32).cuda()
+    pos = torch.cat([torch.arange(n - q, n) for n, q in zip(lengths, q_lens)]).to(torch.int32).cuda()
+    seq = torch.repeat_interleave(torch.arange(2), torch.tensor(q_lens)).to(torch.int32).cuda()
+    ctx = SimpleNamespace(tok_pos=pos, tok_seq=seq, n_tokens=T, n_seqs=2, cu_q=cu, is_decode=False,
+                          kv_len=torch.tensor(lengths, dtype=torch.int32).cuda(), host_q_lens=q_lens, host_kv_lens=lengths,
+                          max_q_len=1500, max_kv_len=2200, extras={})
+    x = rnd(T, (H + 2 * K if form == "plain" else H) * D, dtype=torch.bfloat16, seed=3)
+    R = D // 8
+    outs = []
+    for _ in range(12):
+        out = torch.zeros(T, H * D, dtype=torch.bfloat16, device="cuda")
+        if form == "plain":
+            ops.attention(x, out, KVLayerView(kp, vp, table, None), ctx, H, K, D, D ** -0.5)
+        else:
+            ops.latent_attention_mma(x, out, KVLayerView(kp, None, table, None), ctx, H, D - R, R, D ** -0.5)
+        outs.append(out.view(T, H, D) if form == "plain" else out.view(T, H, D)[..., :D - R])
+    ops.check_tc_status()
+    assert all(torch.equal(o, outs[0]) for o in outs)
+    q = x.view(T, -1, D)[:, :H].double()
+    for b in range(2):
+        at = slice(int(cu[b]), int(cu[b + 1]))
+        keys, values = (p[table[b].long()].transpose(1, 2).reshape(-1, K, D)[:lengths[b]].double()
+                        for p in (kp, vp if form == "plain" else kp))
+        hidden = torch.arange(lengths[b], device="cuda")[None] > pos[at, None]
+        for h in range(H):
+            p = torch.softmax((q[at, h] @ keys[:, h * K // H].T * D ** -0.5).masked_fill(hidden, -math.inf), -1)
+            want = (p @ values[:, h * K // H])[:, :outs[0].shape[-1]]
+            err = (outs[0][at, h].double() - want).norm(dim=1) / want.norm(dim=1)
+            assert err.max().item() < 2.0 ** -6, (b, h)
