@@ -146,13 +146,13 @@ template <int NT> struct F32Shape {
   static_assert(CTAS * (SMEM + 1024) <= 233472, "what a CTA may have");
 };
 
-// CS: the CTAs of a cluster that share a tile, GROUPS / CS runs each; with several, each then adds up its part of the tile
-// through distributed shared memory.  VEC: both operands' rows can be copied 16 bytes at a time.
-template <int NT, bool VEC, int CS>
+// PER: the runs of a CTA: all of them, half of GROUPS or one.  `cs` CTAs then share a tile as a cluster, and each adds up its
+// part of the tile through distributed shared memory.  VEC: both operands' rows can be copied 16 bytes at a time.
+template <int NT, bool VEC, int PER>
 __global__ void __launch_bounds__(F32Shape<NT>::THREADS, F32Shape<NT>::CTAS)
 gemm_f32_nt_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw,
                    const float* __restrict__ bias, float* __restrict__ C, int ldc, int M, int N, int K, int run,
-                   float inv_tau, int n) {
+                   float inv_tau, int n, int cs) {
   using S = F32Shape<NT>;
   constexpr int BLOCKS = S::BLOCKS, RAW = S::RAW, SLOTS = S::SLOTS, PASSES = S::PASSES, STEP = S::ADDERS / 4;
   extern __shared__ unsigned char smem_raw[];
@@ -166,8 +166,10 @@ gemm_f32_nt_kernel(const float* __restrict__ A, int lda, const float* __restrict
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(rest_read + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int rank = (int)(blockIdx.x % CS), share_k = run * (GROUPS / CS);      // the cluster lies along x
-  const int m0 = blockIdx.y * n, n0 = (blockIdx.x / CS) * 128;
+  constexpr bool ALONE = PER == GROUPS;
+  const int rank = ALONE ? 0 : (int)(blockIdx.x % (unsigned)cs);      // the cluster lies along x
+  const int share_k = run * PER;
+  const int m0 = blockIdx.y * n, n0 = (ALONE ? blockIdx.x : blockIdx.x / (unsigned)cs) * 128;
   const int kbegin = min(K, rank * share_k), kend = min(K, kbegin + share_k);
   const int tiles = (kend - kbegin + BK - 1) / BK, per_run = run / BK;
 
@@ -360,13 +362,13 @@ gemm_f32_nt_kernel(const float* __restrict__ A, int lda, const float* __restrict
             at_ld_wait();
             add8(acc[i], d);
           }
-          if (CS == 1 && last && run_index >= GROUPS / 2) {
+          if (ALONE && last && run_index >= GROUPS / 2) {
             ld8(col + 4 * n, d);
             at_ld_wait();
             add8(acc[i], d);
           }
           if (!last) {
-            st8(col + (3 + (CS == 1 && run_index == GROUPS / 2 - 1)) * n, acc[i]);
+            st8(col + (3 + (ALONE && run_index == GROUPS / 2 - 1)) * n, acc[i]);
 #pragma unroll
             for (int e = 0; e < 4; ++e) acc[i][e] = make_float2(0.f, 0.f);
           }
@@ -401,37 +403,38 @@ gemm_f32_nt_kernel(const float* __restrict__ A, int lda, const float* __restrict
   __syncthreads();
   if (warp == S::WARPS)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(S::TMEM_COLS));
-  if (CS > 1) asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-  const int runs = (K + run - 1) / run, share = n * 128 / CS;
+  if (!ALONE) asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   const uint32_t own = at_smem(part);
-  // (the warps that have the fewest registers stay out)
-  const int end = warp < S::WARPS ? (rank + 1) * share : 0;
+  // this CTA's rows of A (the warps that have the fewest registers stay out)
+  const int row_end = (rank + 1) * n / cs, end = warp < S::WARPS ? row_end * 128 : 0;
 #pragma unroll 1
-  for (int e = rank * share + threadIdx.x; e < end; e += 32 * S::WARPS) {
+  for (int e = rank * n / cs * 128 + threadIdx.x; e < end; e += 32 * S::WARPS) {
     const int m = m0 + e / 128, nn = n0 + e % 128;
     if (m >= M || nn >= N) continue;
     float z = part[e];
-    if (CS > 1) {
-      float v[CS];
+    if (!ALONE) {
+      constexpr int MOST = GROUPS / PER;           // CTAs; the first MOST / 2 have the first four runs
+      float v[MOST];
 #pragma unroll
-      for (int g = 0; g < CS; ++g) {
+      for (int g = 0; g < MOST; ++g) {
+        if (g >= cs) continue;
         uint32_t far;
         asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(far) : "r"(own + 4u * e), "r"(g));
         asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v[g]) : "r"(far));
       }
-      float lo = v[0], hi = v[CS / 2];
+      float lo = v[0], hi = v[MOST / 2];
 #pragma unroll
-      for (int g = 1; g < CS / 2; ++g) {
-        if (g < runs) lo += v[g];
-        if (CS / 2 + g < runs) hi += v[CS / 2 + g];
+      for (int g = 1; g < MOST / 2; ++g) {
+        if (g < cs) lo += v[g];
+        if (MOST / 2 + g < cs) hi += v[MOST / 2 + g];
       }
-      z = runs > GROUPS / 2 ? lo + hi : lo;
+      z = cs > MOST / 2 ? lo + hi : lo;
     }
     if (!is_finite(z)) z = plain_dot(A + (size_t)m * lda, W + (size_t)nn * ldw, K, run);
     C[(size_t)m * ldc + nn] = finish(z + (bias ? bias[nn] : 0.f), inv_tau);
   }
   // nobody leaves while its partial sums may still be read
-  if (CS > 1) asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (!ALONE) asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 struct F32Problem {
@@ -439,25 +442,25 @@ struct F32Problem {
   float* C;
   int lda, ldw, ldc, M, N, K, run;
   float inv_tau;
-  int n;
+  int n, cs;
   cudaStream_t stream;
 };
 
-template <int NT, bool VEC, int CS>
+template <int NT, bool VEC, int PER>
 static int launch_f32(const F32Problem& p) {
   constexpr int smem = F32Shape<NT>::SMEM;
-  auto kernel = gemm_f32_nt_kernel<NT, VEC, CS>;
+  auto kernel = gemm_f32_nt_kernel<NT, VEC, PER>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return AB_CUDA_ERR + (int)e;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((p.N + 127) / 128 * CS, (p.M + p.n - 1) / p.n);
+  cfg.gridDim = dim3((p.N + 127) / 128 * p.cs, (p.M + p.n - 1) / p.n);
   cfg.blockDim = dim3(F32Shape<NT>::THREADS);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = p.stream;
   cudaLaunchAttribute attr[2];
-  if (CS > 1) {
+  if (PER < GROUPS) {
     attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
-    attr[cfg.numAttrs].val.clusterDim.x = CS;
+    attr[cfg.numAttrs].val.clusterDim.x = p.cs;
     attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
     ++cfg.numAttrs;
   }
@@ -467,14 +470,56 @@ static int launch_f32(const F32Problem& p) {
     ++cfg.numAttrs;
   }
   cfg.attrs = attr;
-  e = cudaLaunchKernelEx(&cfg, kernel, p.A, p.lda, p.W, p.ldw, p.bias, p.C, p.ldc, p.M, p.N, p.K, p.run, p.inv_tau, p.n);
+  e = cudaLaunchKernelEx(&cfg, kernel, p.A, p.lda, p.W, p.ldw, p.bias, p.C, p.ldc, p.M, p.N, p.K, p.run, p.inv_tau, p.n, p.cs);
   return e == cudaSuccess ? AB_OK : AB_CUDA_ERR + (int)e;
 }
 
+template <int NT, bool VEC>
+static int launch_f32(const F32Problem& p, int per) {
+  return per == GROUPS ? launch_f32<NT, VEC, GROUPS>(p) : per == 1 ? launch_f32<NT, VEC, 1>(p) : launch_f32<NT, VEC, GROUPS / 2>(p);
+}
 template <int NT>
-static int launch_f32(const F32Problem& p, bool vec, int cs) {
-  if (vec) return cs == 1 ? launch_f32<NT, true, 1>(p) : cs == 2 ? launch_f32<NT, true, 2>(p) : launch_f32<NT, true, 8>(p);
-  return cs == 1 ? launch_f32<NT, false, 1>(p) : cs == 2 ? launch_f32<NT, false, 2>(p) : launch_f32<NT, false, 8>(p);
+static int launch_f32(const F32Problem& p, bool vec, int per) {
+  return vec ? launch_f32<NT, true>(p, per) : launch_f32<NT, false>(p, per);
+}
+
+// How a product is cut: k of a run, rows of a tile, the runs of a CTA and the CTAs that share a tile.
+struct F32Plan {
+  int run, n, per, cs;
+};
+static F32Plan plan_f32(int M, int N, int K, int sms) {
+  F32Plan p;
+  p.run = ((K + GROUPS - 1) / GROUPS + BK - 1) / BK * BK;
+  if (p.run < SHORTEST) p.run = SHORTEST;
+  // as few tiles of rows as 128 allow, then as low as they can be
+  // (where a tile is one short run and 64 rows leave processors idle, by 64: 200 rows of 2048x128 11.4 -> 8.7 us)
+  const int top = K <= SHORTEST && (long long)((N + 127) / 128) * ((M + 63) / 64) <= sms ? 64 : 128;
+  const int row_tiles = (M + top - 1) / top;
+  p.n = ((M + row_tiles - 1) / row_tiles + 15) / 16 * 16;
+  const long long tiles = (long long)((N + 127) / 128) * row_tiles;
+  // CTAs of a cluster of 1, 2, .. 8 that run at once on 148 processors, one per processor (what the runtime says)
+  static const int together[GROUPS + 1] = {0, 148, 148, 135, 132, 130, 132, 105, 120};
+  // Runs of a CTA: rounds of CTAs times what one takes.  It starts and ends in about four stages, and in one more with a
+  // cluster or more than 64 rows; where two share a processor, each takes a third longer.  A cluster has as many CTAs as have
+  // a run.  us with all runs / half of them / one in a CTA: one row of 2048x768 20.3 / 15.1 / 6.4, of 512x384 11.3 / - /
+  // 6.4, of 16384x768 20.9 / 20.3 / 24.7; 200 rows of 2048x768 - / 27.7 / 22.2, of 16384x384 43 / - / 74; 333 rows of
+  // 2048x2048 - / 44 / 60.  Of 480 products of 160 to 8,192 k none is more than a tenth slower than with the best of the
+  // three.  (Clusters of two or eight alone, whether or not their CTAs had a run: one row of 2048x768 15.3.)
+  const int runs = (K + p.run - 1) / p.run;
+  p.per = GROUPS;
+  p.cs = 1;
+  long long best = 0;
+  for (int per : {GROUPS, GROUPS / 2, 1}) {
+    if (per == GROUPS && p.n > 96 && runs > GROUPS / 2) continue;      // no room for the second sum of runs
+    const int cs = (runs + per - 1) / per;
+    if (per < GROUPS && cs < 2) continue;                              // nothing to share
+    const long long ctas = tiles * cs, alone = (long long)together[cs ? cs : 1] * sms / 148, at_once = p.n <= 32 ? 2 * alone : alone;
+    const int k = K < p.run * per ? K : p.run * per;
+    long long cost = (ctas + at_once - 1) / at_once * ((k + BK - 1) / BK + (p.n > 64 || cs > 1 ? 5 : 4)) * 10;
+    if (p.n <= 32 && ctas > alone) cost = cost * 13 / 10;
+    if (!best || cost < best) { best = cost; p.per = per; p.cs = cs > 1 ? cs : 1; }
+  }
+  return p;
 }
 
 static int gemm_f32(const float* A, int lda, const float* W, int ldw, const float* bias, float* C, int ldc, int M, int N,
@@ -482,38 +527,26 @@ static int gemm_f32(const float* A, int lda, const float* W, int ldw, const floa
   if (M <= 0 || N <= 0) return AB_OK;
   if (K < 0) return AB_BAD_ARG;
   if ((M + 63) / 64 > 65535) return AB_BAD_ARG;
-  F32Problem p{A, W, bias, C, lda, ldw, ldc, M, N, K, 0, inv_tau, 0, stream};
-  p.run = ((K + GROUPS - 1) / GROUPS + BK - 1) / BK * BK;
-  if (p.run < SHORTEST) p.run = SHORTEST;
   // 16-byte copies where every row of both operands starts on a 16-byte boundary and ends on one
   const bool vec = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)W & 15) == 0;
   int sms = 148, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  // as few tiles of rows as 128 allow, then as low as they can be
-  // (where a tile is one short run and 64 rows leave processors idle, by 64: 200 rows of 2048x128 11.4 -> 8.7 us)
-  const int top = K <= SHORTEST && (long long)((N + 127) / 128) * ((M + 63) / 64) <= sms ? 64 : 128;
-  const int row_tiles = (M + top - 1) / top;
-  p.n = ((M + row_tiles - 1) / row_tiles + 15) / 16 * 16;
-  const long long tiles = (long long)((N + 127) / 128) * row_tiles;
-  const int resident = p.n <= 32 ? 2 * sms : sms;
-  // CTAs per tile: rounds of CTAs times what one takes, in stages of k (it starts and ends in about 8 of them; clusters leave a
-  // tenth of the processors unused).  us with 1 / 2 / 8: one row of 16384x2048 54 / 39 / 54, of 3072x2048 50 / 27 / 13; 200 rows of
-  // 3072x2048 44 / 44 / 59, of 2048x8192 133 / 133 / 112.
-  const long long runs = (K + p.run - 1) / p.run;
-  int cs = 1;
-  long long best = 0;
-  for (int c : {1, 2, 8}) {
-    if (c == 1 && p.n > 96 && runs > GROUPS / 2) continue;      // no room for the second sum of runs
-    if (c > runs && c > 1) continue;
-    const long long at_once = c == 1 ? resident : resident * 9 / 10;
-    const long long cost = (tiles * c + at_once - 1) / at_once * ((runs + c - 1) / c * (p.run / BK) + 8);
-    if (!best || cost < best) { best = cost; cs = c; }
-  }
-  if (p.n <= 16) return launch_f32<16>(p, vec, cs);
-  if (p.n <= 32) return launch_f32<32>(p, vec, cs);
-  if (p.n <= 64) return launch_f32<64>(p, vec, cs);
-  return launch_f32<128>(p, vec, cs);
+  const F32Plan c = plan_f32(M, N, K, sms);
+  const F32Problem p{A, W, bias, C, lda, ldw, ldc, M, N, K, c.run, inv_tau, c.n, c.cs, stream};
+  if (c.n <= 16) return launch_f32<16>(p, vec, c.per);
+  if (c.n <= 32) return launch_f32<32>(p, vec, c.per);
+  if (c.n <= 64) return launch_f32<64>(p, vec, c.per);
+  return launch_f32<128>(p, vec, c.per);
+}
+
+// The plan of a product on 148 processors: k of a run, rows of a tile, runs of a CTA, CTAs of a cluster
+AB_API void ab_gemm_f32_plan(int M, int N, int K, int* out) {
+  const F32Plan p = plan_f32(M, N, K, 148);
+  out[0] = p.run;
+  out[1] = p.n;
+  out[2] = p.per;
+  out[3] = p.cs;
 }
 
 AB_API int ab_gemm_f32_nt(const float* A, int lda, const float* W, int ldw, const float* bias, float* C, int ldc,
