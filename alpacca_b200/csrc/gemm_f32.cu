@@ -16,9 +16,10 @@
 // rows are in the batch: the same token gives the same bits alone and in any batch.  This is the matrix product of the
 // 32-bit path (the reference's float32 path uses BLAS SGEMM, alpacca/tensor.py:91-97).
 //
-// A number that is not finite, or above the largest bfloat16, splits into infinities and NaNs; so do the sums.  An
-// output that comes out not finite is therefore formed again by plain multiply-adds (`plain_dot`): what the sum gives
-// in 32 bits, infinities included.
+// The parts are those of 2^16 times a number, so that the smallest number's last bit is one of a bfloat16 too, and outputs
+// are multiplied by 2^-32: powers of two, which change no other bit.  A number of 2^112 or more splits into infinities and
+// NaNs, an output of 2^96 or more overflows.  An output that comes out not finite is therefore formed again by plain
+// multiply-adds (`plain_dot`): what the sum gives in 32 bits, infinities included.
 //
 // A tile is 128 rows of W (the 128 rows of an MMA) by n <= 128 rows of A.  Splitting warps bring both operands' 32-bit rows
 // by cp.async into a ring in shared memory (each thread only what it splits itself, so nobody waits for anybody), split
@@ -94,9 +95,14 @@ __device__ __forceinline__ void less(uint32_t& a, uint32_t& b, uint32_t pa, uint
   asm("{\n\t.reg .b64 x, p;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 p, {%2, %3};\n\t"
       "fma.rn.f32x2 x, p, %4, x;\n\tmov.b64 {%0, %1}, x;\n\t}" : "+r"(a), "+r"(b) : "r"(pa), "r"(pb), "l"(0xbf800000bf800000ull));
 }
-// Two numbers (their bits) to two words of parts, the first in the lower half.  Rounded, so that the rest has either sign and
-// the three products left out cancel; what is left for l is at most eight bits.
+// Two numbers (their bits) to two words of parts of 2^16 times them, the first in the lower half.  Rounded, so that the rest
+// has either sign and the three products left out cancel; what is left for l is at most eight bits.  Below 2^-110 a number's
+// last bits would lie under 2^-133, the last bit of bfloat16: times 2^16 the smallest number's last bit lies on it.
+#define SCALE_BITS 0x4780000047800000ull      // 2^16, twice
+#define UNSCALE 0x1p-32f                      // what a product is multiplied by in the end
 __device__ __forceinline__ void split2(uint32_t a, uint32_t b, uint32_t& h, uint32_t& m, uint32_t& l) {
+  asm("{\n\t.reg .b64 x;\n\tmov.b64 x, {%0, %1};\n\tmul.rn.f32x2 x, x, %2;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "+r"(a), "+r"(b) : "l"(SCALE_BITS));
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(h) : "f"(__uint_as_float(b)), "f"(__uint_as_float(a)));
   less(a, b, h << 16, h & 0xffff0000u);
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(m) : "f"(__uint_as_float(b)), "f"(__uint_as_float(a)));
@@ -430,6 +436,7 @@ gemm_f32_nt_kernel(const float* __restrict__ A, int lda, const float* __restrict
       }
       z = cs > MOST / 2 ? lo + hi : lo;
     }
+    z *= UNSCALE;
     if (!is_finite(z)) z = plain_dot(A + (size_t)m * lda, W + (size_t)nn * ldw, K, run);
     C[(size_t)m * ldc + nn] = finish(z + (bias ? bias[nn] : 0.f), inv_tau);
   }

@@ -798,3 +798,19 @@ def test_prompt_attention_waits_for_its_last_products(form, H, K, D):
             want = (p @ values[:, h * K // H])[:, :outs[0].shape[-1]]
             err = (outs[0][at, h].double() - want).norm(dim=1) / want.norm(dim=1)
             assert err.max().item() < 2.0 ** -6, (b, h)
+
+
+@pytest.mark.parametrize("M,K", [(1, 96), (16, 2048), (40, 1100), (130, 513)])
+@pytest.mark.parametrize("small,large", [(-105, 100), (-112, 100), (-120, 100), (-126, 120), (-140, 110), (-149, 60), (-65, -65), (-75, -70)])
+def test_gemm_f32_small_numbers(M, K, small, large):
+    """Numbers whose last bits lie below bfloat16's smallest, down to subnormal ones, times large ones, and products that are
+    subnormal themselves.  Bound: that of the tiles' test, and half a last place of the smallest number for the result."""
+    from alpacca_b200 import ops
+    N = 150
+    a, w = (rnd(M, K, seed=1).double() * 2.0 ** small).float(), (rnd(N, K, seed=2).double() * 2.0 ** large).float()
+    a[:, ::5] = 0.0
+    out = torch.empty(M, N, device="cuda")
+    ops.gemm_f32(a, w, out)
+    want = a.double() @ w.double().T
+    bound = 2.0 ** -22 * a.double().norm(dim=1)[:, None] * w.double().norm(dim=1)[None] + 2.0 ** -150
+    assert want.abs().max() > 0 and ((out.double() - want).abs() <= bound).all()
