@@ -85,6 +85,10 @@ __device__ __forceinline__ void add8(float2* a, const float2* v) {
     asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 y, {%2, %3};\n\tadd.rn.f32x2 x, x, y;\n\t"
         "mov.b64 {%0, %1}, x;\n\t}" : "+f"(a[i].x), "+f"(a[i].y) : "f"(v[i].x), "f"(v[i].y));
 }
+__device__ __forceinline__ void fma2(float2& s, float ax, float ay, float bx, float by) {      // s += (ax bx, ay by)
+  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%0, %1};\n\t"
+      "fma.rn.f32x2 z, x, y, z;\n\tmov.b64 {%0, %1}, z;\n\t}" : "+f"(s.x), "+f"(s.y) : "f"(ax), "f"(ay), "f"(bx), "f"(by));
+}
 __device__ __forceinline__ void st8(uint32_t taddr, const float2* v) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(__float_as_uint(v[0].x)),
                "r"(__float_as_uint(v[0].y)), "r"(__float_as_uint(v[1].x)), "r"(__float_as_uint(v[1].y)),
@@ -444,6 +448,76 @@ gemm_f32_nt_kernel(const float* __restrict__ A, int lda, const float* __restrict
   if (!ALONE) asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+// Products of few k, by plain multiply-adds: two chains per output, over its even and its odd k, added at the end.  Below
+// SHORT_K the several roundings and the parts left out weigh more than the few roundings of the chains, so these take no
+// tensor core.  Error against 64 bits, root mean square over the result's, split / chains, x 1e-9: one k 26.0 / 25.4, numbers
+// of very unlike sizes 16 k 64.8 / 46.6, 32 k 74.0 / 64.7, 48 k 74.2 / 74.5; largest over the sum of |a| |w|, one k 88 / 60.
+// All k of a tile lie in shared memory at once, [row][k], KP floats apart (eight neighbouring threads' 16 bytes meet every
+// bank once); two k side by side are one fma.rn.f32x2.  Bound by the latency of its few steps.  us split / chains: one row of
+// 2048x16 3.2 / 1.9, 48 rows 5.1 / 2.9, 333 rows 5.7 / 3.6; of 16384x32 3.3 / 2.4, 5.4 / 4.8, 24.6 / 14.7; of 2048x47
+// 4.8 / 3.2, 7.0 / 5.0, 7.9 / 7.2.
+#define SHORT_K 48
+template <int BM, int BN, int TM, int TN>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN))
+gemm_f32_short_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw, const float* __restrict__ bias,
+                      float* __restrict__ C, int ldc, int M, int N, int K, float inv_tau, bool vec) {
+  constexpr int NX = BN / TN, NY = BM / TM, T = NX * NY, KP = SHORT_K + 4;
+  __shared__ __align__(16) float smem[(BM + BN) * KP];
+  pdl_wait();
+  pdl_trigger();
+  const int tx = threadIdx.x % NX, ty = threadIdx.x / NX;
+  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+  // rows of A, then of W, in pieces of four k, zeros past the matrices: 4, 8 or 16 threads to a row (a division per piece
+  // cost 0.7 us)
+  const int shift = K <= 16 ? 2 : K <= 32 ? 3 : 4, k0 = (threadIdx.x & ((1 << shift) - 1)) * 4;
+  if (k0 < K) {
+#pragma unroll 4
+    for (int r = threadIdx.x >> shift; r < BM + BN; r += T >> shift) {
+      const bool in = r < BM ? m0 + r < M : n0 + r - BM < N;
+      const float* src = !in ? A : (r < BM ? A + (size_t)(m0 + r) * lda : W + (size_t)(n0 + r - BM) * ldw) + k0;
+      const uint32_t dst = at_smem(smem + r * KP + k0);
+      if (vec) {
+        cp_async16(dst, src, in ? 16 : 0);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) cp_async4(dst + 4 * e, in && k0 + e < K ? src + e : A, in && k0 + e < K ? 4 : 0);
+      }
+    }
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+  float2 acc[TM][TN];
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j) acc[i][j] = make_float2(0.f, 0.f);
+#pragma unroll 4
+  for (int k = 0; k < K; k += 4) {
+    float4 a[TM], w[TN];
+#pragma unroll
+    for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const float4*>(smem + (ty + NY * i) * KP + k);
+#pragma unroll
+    for (int j = 0; j < TN; ++j) w[j] = *reinterpret_cast<const float4*>(smem + (BM + tx + NX * j) * KP + k);
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int j = 0; j < TN; ++j) {
+        fma2(acc[i][j], a[i].x, a[i].y, w[j].x, w[j].y);
+        fma2(acc[i][j], a[i].z, a[i].w, w[j].z, w[j].w);
+      }
+  }
+#pragma unroll
+  for (int i = 0; i < TM; ++i) {
+    const int m = m0 + ty + NY * i;
+    if (m >= M) continue;
+#pragma unroll
+    for (int j = 0; j < TN; ++j) {
+      const int nn = n0 + tx + NX * j;
+      if (nn < N) C[(size_t)m * ldc + nn] = finish(acc[i][j].x + acc[i][j].y + (bias ? bias[nn] : 0.f), inv_tau);
+    }
+  }
+}
+
 struct F32Problem {
   const float *A, *W, *bias;
   float* C;
@@ -529,6 +603,14 @@ static F32Plan plan_f32(int M, int N, int K, int sms) {
   return p;
 }
 
+template <int BM, int BN, int TM, int TN>
+static int launch_short(const F32Problem& p, bool vec) {
+  const cudaError_t e = ab_launch(gemm_f32_short_kernel<BM, BN, TM, TN>, dim3((p.N + BN - 1) / BN, (p.M + BM - 1) / BM),
+                                  dim3((BM / TM) * (BN / TN)), 0, p.stream, p.A, p.lda, p.W, p.ldw, p.bias, p.C, p.ldc, p.M, p.N, p.K,
+                                  p.inv_tau, vec);
+  return e == cudaSuccess ? AB_OK : AB_CUDA_ERR + (int)e;
+}
+
 static int gemm_f32(const float* A, int lda, const float* W, int ldw, const float* bias, float* C, int ldc, int M, int N,
                     int K, float inv_tau, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return AB_OK;
@@ -539,8 +621,18 @@ static int gemm_f32(const float* A, int lda, const float* W, int ldw, const floa
   int sms = 148, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  F32Problem p{A, W, bias, C, lda, ldw, ldc, M, N, K, 0, inv_tau, 0, 0, stream};
+  if (K < SHORT_K) {
+    // few rows: as low a tile as holds them; more: the tile that pads fewer, of equals the square one
+    if (M <= 8) return launch_short<8, 128, 8, 1>(p, vec);
+    if (M <= 16 || (M <= 32 && N <= 8192)) return launch_short<16, 128, 8, 2>(p, vec);
+    const long long low = (M + 31) / 32 * 32LL, square = (M + 63) / 64 * 64LL;
+    return low < square * 0.97 && low / 32 <= 65535 ? launch_short<32, 128, 8, 4>(p, vec) : launch_short<64, 64, 8, 4>(p, vec);
+  }
   const F32Plan c = plan_f32(M, N, K, sms);
-  const F32Problem p{A, W, bias, C, lda, ldw, ldc, M, N, K, c.run, inv_tau, c.n, c.cs, stream};
+  p.run = c.run;
+  p.n = c.n;
+  p.cs = c.cs;
   if (c.n <= 16) return launch_f32<16>(p, vec, c.per);
   if (c.n <= 32) return launch_f32<32>(p, vec, c.per);
   if (c.n <= 64) return launch_f32<64>(p, vec, c.per);

@@ -814,3 +814,22 @@ def test_gemm_f32_small_numbers(M, K, small, large):
     want = a.double() @ w.double().T
     bound = 2.0 ** -22 * a.double().norm(dim=1)[:, None] * w.double().norm(dim=1)[None] + 2.0 ** -150
     assert want.abs().max() > 0 and ((out.double() - want).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("M,N", [(1, 40), (16, 129), (33, 300), (70, 64), (200, 1000)])
+@pytest.mark.parametrize("K", [1, 2, 5, 16, 31, 40, 47])
+def test_gemm_f32_of_few_k_rounds_as_its_chains_do(M, N, K):
+    """Few k are two chains of multiply-adds, over the even and the odd k, added at the end: formed here in 64 bits (a product of
+    two 32-bit numbers is exact there) and rounded after every step.  Only where that rounds twice may the last bit differ."""
+    from alpacca_b200 import ops
+    a, w = rnd(M, K, seed=1), rnd(N, K, seed=2)
+    a *= torch.exp2(torch.randint(-20, 20, (M, K), generator=torch.Generator().manual_seed(3)).float()).cuda()
+    out, out1 = torch.empty(M, N, device="cuda"), torch.empty(1, N, device="cuda")
+    ops.gemm_f32(a, w, out)
+    ops.gemm_f32(a[M // 2:M // 2 + 1].contiguous(), w, out1)
+    chain = [torch.zeros(M, N, device="cuda"), torch.zeros(M, N, device="cuda")]
+    for k in range(K):
+        chain[k % 2] = (chain[k % 2].double() + a[:, k, None].double() * w[None, :, k].double()).float()
+    want = chain[0] + chain[1]
+    assert torch.equal(out1[0], out[M // 2])
+    assert (out != want).float().mean().item() < 1e-3 and (out - want).abs().max() <= 2.0 ** -20 * want.abs().max()
