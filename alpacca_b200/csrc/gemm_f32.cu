@@ -19,7 +19,7 @@
 // The parts are those of 2^16 times a number, so that the smallest number's last bit is one of a bfloat16 too, and outputs
 // are multiplied by 2^-32: powers of two, which change no other bit.  A number of 2^112 or more splits into infinities and
 // NaNs, an output of 2^96 or more overflows.  An output that comes out not finite is therefore formed again by plain
-// multiply-adds (`plain_dot`): what the sum gives in 32 bits, infinities included.
+// multiply-adds (`plain_rows`): what the sum gives in 32 bits, infinities included.
 //
 // A tile is 128 rows of W (the 128 rows of an MMA) by n <= 128 rows of A.  Splitting warps bring both operands' 32-bit rows
 // by cp.async into a ring in shared memory (each thread only what it splits itself, so nobody waits for anybody), split
@@ -34,7 +34,7 @@
 // conversion instruction (the same); two leading accumulators (one row 0.8 us slower a product).
 //
 // Every wait on an mbarrier is bounded; a thread that gives up leaves a code in `gemm_f32_stuck`, all roles fall through
-// to the end, where TMEM is given back, and the outputs are NaN until `plain_dot` has formed them.
+// to the end, where TMEM is given back, and the outputs are NaN until `plain_rows` has formed them.
 #include "attention_tc.cuh"
 #include "common.cuh"
 #include "launch.cuh"
@@ -120,17 +120,92 @@ __device__ __forceinline__ float finish(float z, float inv_tau) {
   const float sp = -z > 20.f ? -z : log1pf(expf(-z));      // -log sigmoid(z)
   return expf(-sp * inv_tau);
 }
-// an output by plain multiply-adds, runs in ascending order: for sums that the split numbers cannot form
-__device__ __noinline__ float plain_dot(const float* __restrict__ a, const float* __restrict__ w, int K, int run) {
-  float tot = 0.f;
-  for (int k0 = 0; k0 < K; k0 += run) {
-    float s = 0.f;
-    for (int k = k0; k < min(K, k0 + run); ++k) s = fmaf(a[k], w[k], s);
-    tot = k0 ? tot + s : s;
-  }
-  return tot;
-}
 __device__ __forceinline__ bool is_finite(float z) { return (__float_as_uint(z) & 0x7f800000u) != 0x7f800000u; }
+
+// Outputs that the split numbers cannot form, those marked by a number that is not finite in `part` ([n][128], rows of A by
+// rows of W), by plain multiply-adds: rows row .. row_end of A from `a`, the `cols` rows of W from `w`, the runs of k in
+// ascending order.  T threads (a thread has a column and FALL rows at a time), 32 k after the other by cp.async into `room`.
+// A function of its own with few rows a thread: inlined, or with eight rows, it took registers from the loops before it
+// (333 rows of 16384x2048 without such outputs 267 -> 272 us).  us with a thread per output that reads both rows from global
+// memory / this / the multiply-adds of before: one row of 16384x2048 with a NaN 321 / 115 / 38, one such row of 333
+// 516 / 354 / 572, all of 48 11,500 / 426 / 119, all of 333 47,000 / 2,630 / 574; a row of W with a NaN 819 / 444 / 572, of
+// 2048x8192 (half the runs in a CTA: every row of the tile again) 726 / 1,155 / 315.
+#define FALL 4
+#define FALL_BUFFERS 4
+template <int T> struct Fall {
+  static constexpr int PASS = T / 128 * FALL;                       // rows at a time
+  static constexpr int KP = BK + 4;                                 // eight neighbouring threads' 16 bytes meet every bank once
+  static constexpr int BUFFER = (128 + PASS) * KP;                  // floats
+};
+template <int T, bool VEC>
+__device__ __noinline__ void plain_rows(const float* __restrict__ a, int lda, const float* __restrict__ w, int ldw,
+                                           const float* __restrict__ bias, float* __restrict__ c, int ldc, int row, int row_end,
+                                           int cols, int K, int run, float inv_tau, const float* part, float* room) {
+  using F = Fall<T>;
+  const int col = threadIdx.x & 127, first = (threadIdx.x >> 7) * FALL;
+#pragma unroll 1
+  for (; row < row_end; row += F::PASS) {
+    uint32_t bad = 0;
+#pragma unroll
+    for (int i = 0; i < FALL; ++i)
+      if (first < F::PASS && row + first + i < row_end && col < cols && !is_finite(part[(row + first + i) * 128 + col])) bad |= 1u << i;
+    uint32_t any;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbarrier.cta.red.or.pred p, 1, %2, q;\n\t"
+                 "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(any) : "r"(bad), "n"(T) : "memory");
+    if (!any) continue;
+    auto stage = [&](int t) {                      // 32 k from t * BK on, an empty group past the end
+      if (t * BK < K) {
+        float* to = room + t % FALL_BUFFERS * F::BUFFER;
+        constexpr int E = VEC ? 4 : 1;
+#pragma unroll 1
+        for (int i = threadIdx.x; i < (128 + F::PASS) * (BK / E); i += T) {
+          const int r = i / (BK / E), k = t * BK + i % (BK / E) * E;
+          const bool in = k < K && (r < 128 ? r < cols : row + r - 128 < row_end);
+          const float* from = !in ? a : (r < 128 ? w + (size_t)r * ldw : a + (size_t)(row + r - 128) * lda) + k;
+          const uint32_t at = at_smem(to + r * F::KP + i % (BK / E) * E);
+          if (VEC) cp_async16(at, from, in ? 16 : 0);
+          else cp_async4(at, from, in ? 4 : 0);
+        }
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    float sum[FALL], tot[FALL];
+#pragma unroll
+    for (int i = 0; i < FALL; ++i) sum[i] = tot[i] = 0.f;
+#pragma unroll 1
+    for (int t = 0; t < FALL_BUFFERS - 1; ++t) stage(t);
+#pragma unroll 1
+    for (int t = 0, k0 = 0; k0 < K; ++t, k0 += BK) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(FALL_BUFFERS - 2) : "memory");
+      asm volatile("barrier.cta.sync 1, %0;" ::"n"(T) : "memory");      // these k are there for all, those before are read by all
+      stage(t + FALL_BUFFERS - 1);
+      if (__any_sync(0xffffffffu, bad)) {
+        const float* from = room + t % FALL_BUFFERS * F::BUFFER;
+#pragma unroll 2
+        for (int k = 0; k < BK; k += 4) {
+          const float4 y = *reinterpret_cast<const float4*>(from + col * F::KP + k);
+#pragma unroll
+          for (int i = 0; i < FALL; ++i) {
+            const float4 x = *reinterpret_cast<const float4*>(from + (128 + first + i) * F::KP + k);
+            sum[i] = fmaf(x.w, y.w, fmaf(x.z, y.z, fmaf(x.y, y.y, fmaf(x.x, y.x, sum[i]))));
+          }
+        }
+        if ((k0 + BK) % run == 0 || k0 + BK >= K) {
+#pragma unroll
+          for (int i = 0; i < FALL; ++i) {
+            tot[i] = k0 < run ? sum[i] : tot[i] + sum[i];
+            sum[i] = 0.f;
+          }
+        }
+      }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    asm volatile("barrier.cta.sync 1, %0;" ::"n"(T) : "memory");        // the buffers may be filled again
+#pragma unroll
+    for (int i = 0; i < FALL; ++i)
+      if (bad >> i & 1) c[(size_t)(row + first + i) * ldc + col] = finish(tot[i] + (bias ? bias[col] : 0.f), inv_tau);
+  }
+}
 
 // NT: the most rows of A that a tile can hold; `n` of them are this launch's (a multiple of 16).
 template <int NT> struct F32Shape {
@@ -152,7 +227,8 @@ template <int NT> struct F32Shape {
   static constexpr int SMEM = BAR_OFF + 128 + 1024 /*alignment*/;
   static constexpr int CTAS = NT <= 32 ? 2 : 1;                     // per processor
   static constexpr int TMEM_COLS = NT <= 16 ? 128 : NT <= 32 ? 256 : 512;      // four times n of them used, or five times
-  static_assert(BAR_OFF >= 128 * NT * 4, "the partial sums take the tiles' place");
+  static_assert(BAR_OFF >= 128 * NT * 4 + FALL_BUFFERS * Fall<32 * WARPS>::BUFFER * 4, "the partial sums take the tiles' place");
+  static_assert(!UNEQUAL || (THREADS * 80 == 128 * 40 + 32 * SPLITTERS * 72 + 32 * ADDERS * 112), "registers by role");
   static_assert(CTAS * (SMEM + 1024) <= 233472, "what a CTA may have");
 };
 
@@ -174,6 +250,7 @@ gemm_f32_nt_kernel(const float* __restrict__ A, int lda, const float* __restrict
   uint64_t* lead_read = done + SLOTS;            // a stage's leading sums have been read
   uint64_t* rest_read = lead_read + 1;           // a run's other sums have been read
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(rest_read + 1);
+  volatile uint32_t* marked = tmem_slot + 1;     // whether this CTA's part of the outputs has some to be formed again
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr bool ALONE = PER == GROUPS;
@@ -193,6 +270,7 @@ gemm_f32_nt_kernel(const float* __restrict__ A, int lda, const float* __restrict
     for (int i = 0; i < SLOTS; ++i) { at_bar_init(full + i, S::SPLITTERS); at_bar_init(done + i, 1); }
     at_bar_init(lead_read, S::ADDERS);
     at_bar_init(rest_read, S::ADDERS);
+    *marked = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == S::WARPS) {
@@ -209,6 +287,9 @@ gemm_f32_nt_kernel(const float* __restrict__ A, int lda, const float* __restrict
   bool ok = true;
   // an adding warp's columns (rows of A): blocks first, first + STEP, ..
   const int first = STEP == 2 ? (warp >> 2) & 1 : 0, blocks = n / 8;
+  // In the end every warp has the registers of the launch again, the others behind this barrier only: the adding warps have
+  // then taken and given back theirs (warps that took theirs back before would leave too few for them, and all would wait).
+  auto roles_end = [] { asm volatile("barrier.cta.sync 2, %0;" ::"n"(S::THREADS) : "memory"); };
   float* part = reinterpret_cast<float*>(base);  // [n][128]: the sums, once nothing reads or writes the stages any more
   if (warp >= S::WARPS) {
     if (S::UNEQUAL) asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
@@ -240,6 +321,11 @@ gemm_f32_nt_kernel(const float* __restrict__ A, int lda, const float* __restrict
         if (++s == SLOTS) { s = 0; phase ^= 1; }
       }
       if (!ok) atomicExch(&gemm_f32_stuck, 41);
+    }
+    if (S::UNEQUAL) {
+      __syncwarp();
+      roles_end();
+      asm volatile("setmaxnreg.inc.sync.aligned.u32 80;");
     }
   } else if (warp < S::SPLITTERS) {
     if (S::UNEQUAL) asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
@@ -329,6 +415,11 @@ gemm_f32_nt_kernel(const float* __restrict__ A, int lda, const float* __restrict
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     if (!ok && lane == 0) atomicExch(&gemm_f32_stuck, 42);
+    if (S::UNEQUAL) {
+      __syncwarp();
+      roles_end();
+      asm volatile("setmaxnreg.inc.sync.aligned.u32 80;");
+    }
   } else {
     if (S::UNEQUAL) asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
     const uint32_t at = tmem + ((uint32_t)((warp & 3) * 32) << 16) + first * 8;     // its lanes of TMEM: rows of W
@@ -408,6 +499,10 @@ gemm_f32_nt_kernel(const float* __restrict__ A, int lda, const float* __restrict
           mine[(STEP * 8 * i + 2 * e) * 128] = ok ? acc[i][e].x : spoilt;
           mine[(STEP * 8 * i + 2 * e + 1) * 128] = ok ? acc[i][e].y : spoilt;
         }
+    if (S::UNEQUAL) {
+      asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
+      roles_end();
+    }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -415,7 +510,8 @@ gemm_f32_nt_kernel(const float* __restrict__ A, int lda, const float* __restrict
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(S::TMEM_COLS));
   if (!ALONE) asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   const uint32_t own = at_smem(part);
-  // this CTA's rows of A (the warps that have the fewest registers stay out)
+  // this CTA's rows of A (the MMA's warps stay out)
+  uint32_t bad = 0;
   const int row_end = (rank + 1) * n / cs, end = warp < S::WARPS ? row_end * 128 : 0;
 #pragma unroll 1
   for (int e = rank * n / cs * 128 + threadIdx.x; e < end; e += 32 * S::WARPS) {
@@ -441,11 +537,30 @@ gemm_f32_nt_kernel(const float* __restrict__ A, int lda, const float* __restrict
       z = cs > MOST / 2 ? lo + hi : lo;
     }
     z *= UNSCALE;
-    if (!is_finite(z)) z = plain_dot(A + (size_t)m * lda, W + (size_t)nn * ldw, K, run);
-    C[(size_t)m * ldc + nn] = finish(z + (bias ? bias[nn] : 0.f), inv_tau);
+    if (is_finite(z)) {
+      C[(size_t)m * ldc + nn] = finish(z + (bias ? bias[nn] : 0.f), inv_tau);
+    } else {
+      part[e] = z;                                 // a mark (nobody else reads this CTA's own part of its sums)
+      bad = 1;
+    }
   }
-  // nobody leaves while its partial sums may still be read
-  if (!ALONE) asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  bool again;
+  if (ALONE) {
+    if (warp >= S::WARPS) return;
+    uint32_t any;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbarrier.cta.red.or.pred p, 1, %2, q;\n\t"
+                 "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(any) : "r"(bad), "n"(32 * S::WARPS) : "memory");
+    again = any;
+  } else {
+    if (bad) *marked = 1;
+    // nobody leaves while its partial sums may still be read
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    again = *marked && warp < S::WARPS;
+  }
+  if (again)
+    plain_rows<32 * S::WARPS, VEC>(A + (size_t)m0 * lda, lda, W + (size_t)n0 * ldw, ldw, bias ? bias + n0 : nullptr,
+                                             C + (size_t)m0 * ldc + n0, ldc, rank * n / cs, min(row_end, M - m0), min(128, N - n0),
+                                             K, run, inv_tau, part, part + n * 128);
 }
 
 // Products of few k, by plain multiply-adds: two chains per output, over its even and its odd k, added at the end.  Below
@@ -533,6 +648,10 @@ static int launch_f32(const F32Problem& p) {
   auto kernel = gemm_f32_nt_kernel<NT, VEC, PER>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return AB_CUDA_ERR + (int)e;
+  if (F32Shape<NT>::UNEQUAL) {                     // the roles' registers are shares of the launch's: with fewer they would wait
+    static const int regs = [&] { cudaFuncAttributes a; return cudaFuncGetAttributes(&a, kernel) == cudaSuccess ? a.numRegs : 0; }();
+    if (regs != 80) return AB_BAD_ARG;
+  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((p.N + 127) / 128 * p.cs, (p.M + p.n - 1) / p.n);
   cfg.blockDim = dim3(F32Shape<NT>::THREADS);

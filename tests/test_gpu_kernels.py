@@ -833,3 +833,36 @@ def test_gemm_f32_of_few_k_rounds_as_its_chains_do(M, N, K):
     want = chain[0] + chain[1]
     assert torch.equal(out1[0], out[M // 2])
     assert (out != want).float().mean().item() < 1e-3 and (out - want).abs().max() <= 2.0 ** -20 * want.abs().max()
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 300, 2048), (16, 129, 96), (20, 300, 513), (33, 40, 250), (60, 2100, 2048), (97, 300, 1100),
+                                   (130, 20000, 260), (200, 150, 64), (256, 2100, 2048)])
+@pytest.mark.parametrize("every", [False, True])
+def test_gemm_f32_forms_what_is_not_finite_again(M, N, K, every):
+    """Rows of either operand with an infinity or a NaN, and a row whose sums are beyond 2^96, on every tile height, alone and
+    shared by clusters: the former give what 64-bit sums give, the latter keep the tiles' test's bound, all others their bits.
+    `every`: each row of A has a NaN or an infinity."""
+    from alpacca_b200 import ops
+    a, w = rnd(M, K, seed=1), rnd(N, K, seed=2).abs()
+    clean, out = torch.empty(M, N, device="cuda"), torch.full((M + 1, N), 7.0, device="cuda")
+    ops.gemm_f32(a, w, clean)
+    w[N // 3, K // 2], w[N - 1, 0] = float("inf"), float("nan")
+    touched = torch.zeros(M, dtype=torch.bool, device="cuda")
+    touched[M // 2] = True
+    a[M // 2] *= 2.0 ** 98
+    if M > 2:
+        a[0, K - 1], a[M - 1, 3] = float("-inf"), float("nan")
+        touched[0] = touched[M - 1] = True
+    if every:
+        a[::2, 1], a[1::2, K // 3], touched[:] = float("nan"), float("inf"), True
+    ops.gemm_f32(a, w, out, n_rows=M)
+    want = a.double() @ w.double().T
+    got = out[:M]
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isposinf(), want.isposinf()) and (out[M] == 7.0).all()
+    assert torch.equal(got.isneginf(), want.isneginf())
+    finite = want.isfinite()
+    bound = 2.0 ** -22 * a.double().nan_to_num(0, 0, 0).norm(dim=1)[:, None] * w.double().nan_to_num(0, 0, 0).norm(dim=1)[None]
+    assert ((got.double() - want).abs() <= bound)[finite].all()
+    same = finite & ~touched[:, None]
+    assert torch.equal(got[same], clean[same])
+    assert ops.gemm_f32_status() == 0
