@@ -93,8 +93,9 @@ __global__ void attention_simt_kernel(const T* __restrict__ q, int q_stride, T* 
 #pragma unroll
     for (int o = 4; o < 32; o <<= 1) m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, o));
     m_new = fmaxf(m, m_new);
-    const float corr = expf(m - m_new);              // exp(-inf) = 0 on the first run
-    const float p = expf(score - m_new);
+    // a run without a score above -inf changes nothing (before the first such score all maxima are -inf)
+    const float corr = m == m_new ? 1.f : expf(m - m_new);
+    const float p = score == -INFINITY ? 0.f : expf(score - m_new);
     float sum = p;
 #pragma unroll
     for (int o = 4; o < 32; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);

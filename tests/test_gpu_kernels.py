@@ -866,3 +866,37 @@ def test_gemm_f32_forms_what_is_not_finite_again(M, N, K, every):
     same = finite & ~touched[:, None]
     assert torch.equal(got[same], clean[same])
     assert ops.gemm_f32_status() == 0
+
+
+@pytest.mark.parametrize("dtype,H,K,D", [("float32", 4, 1, 64), ("float32", 16, 2, 128), ("float32", 3, 3, 72), ("bfloat16", 6, 2, 72)])
+@pytest.mark.parametrize("window", [0, 30])
+def test_attention_32bit_of_scores_of_minus_infinity(dtype, H, K, D, window):
+    """Keys whose score is -inf get no weight, also where they are the first ones, a whole run of eight or all but one; a row that
+    sees no others is not a number.  The same in every form of the kernel, and what 64-bit arithmetic gives."""
+    from alpacca_b200 import ops
+    lengths, q_lens = [70, 20, 9], [70, 20, 9]
+    table, kp, vp = make_paged(lengths, 5, K, D, DT[dtype], seed=2)
+    ks = [rnd(n, K, D, dtype=DT[dtype], seed=4 + b) for b, n in enumerate(lengths)]
+    vs = [rnd(n, K, D, dtype=DT[dtype], seed=7 + b) for b, n in enumerate(lengths)]
+    for b, gone in enumerate([list(range(17)) + list(range(24, 40)) + [55], list(range(19)), [8]]):
+        ks[b][gone, :, 0] = float("-inf")            # every query is positive there
+        fill_cache(table.cpu(), kp, vp, b, ks[b], vs[b])
+    T = sum(q_lens)
+    qkv = rnd(T, (H + 2 * K) * D, dtype=DT[dtype], seed=3)
+    qkv.view(T, -1, D)[:, :, 0] = qkv.view(T, -1, D)[:, :, 0].abs() + 0.1
+    pos = torch.cat([torch.arange(n) for n in lengths]).to(torch.int32).cuda()
+    seq = torch.repeat_interleave(torch.arange(3), torch.tensor(q_lens)).to(torch.int32).cuda()
+    cu = torch.tensor([0, 70, 90, 99], dtype=torch.int32).cuda()
+    outs = []
+    for form in ({}, {"cu_q": cu}, {"single": True}):
+        out = torch.empty(T, H * D, dtype=DT[dtype], device="cuda")
+        ops.attention_simt(qkv, out, kp, vp, table, pos, seq, T, H, K, D, D ** -0.5, window, **form)
+        outs.append(out.float().nan_to_num(9.0))
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    q = qkv.double().cpu().view(T, -1, D)[:, :H]
+    t0 = 0
+    for b, n in enumerate(lengths):
+        want = ref_attention(q[t0:t0 + n], ks[b].double().cpu(), vs[b].double().cpu(), pos[t0:t0 + n].cpu(), D ** -0.5, window)
+        assert want.isnan().any() == (b < 2) and not want.isnan().all()
+        close(outs[0][t0:t0 + n].view(n, H, D), want.nan_to_num(9.0), dtype, f"sequence {b}")
+        t0 += n
