@@ -7,21 +7,24 @@
 //   score_s = (q . k_s) * scale  for lo <= s <= p   (alpacca/model.py:447-467)
 //   out = sum_s softmax(score)_s * v_s
 // with lo = 0, or p - window + 1 when a window is given.  The softmax is the
-// running (online) form, eight keys at a time in key order; nothing is shared
-// between warps, so a token's result does not depend on the rest of the batch.
+// running (online) form, eight keys at a time in key order; a token's result
+// does not depend on the rest of the batch.
 //
-// Bound by latency: a warp's keys follow one another.  One key at a time is five
-// dependent shuffles, two exponentials and a load that nothing overlaps; eight at
-// a time are eight loads in flight, nine shuffles for their sums and one rescaling.
+// Row by row (attention_simt_kernel): bound by latency, a warp's keys follow one
+// another.  One key at a time is five dependent shuffles, two exponentials and a
+// load that nothing overlaps; eight at a time are eight loads in flight, nine
+// shuffles for their sums and one rescaling.
 // 333 tokens, 32 heads of 64 on 8, float32: 281 -> 169 us.
 //
-// Query heads that come in fours per KV head (attention_rows_kernel): a block takes four heads of eight tokens, a token per warp,
-// and brings 32 keys and values at a time to shared memory, by cp.async, the next 32 under the work on these.  For the scores
-// a lane has a key and forms its four products with the heads; the softmax is that of four runs of eight lanes; for the
-// values a lane has its dimensions.  Every sum is formed in the order of the kernel above, operation by operation, so a row's
-// bits do not depend on which of the two ran.  Bound by instructions (about nine per head and key and 32 lanes).  us one
-// warp per row / this: 333 tokens, 32 heads of 64 on 8, 156 / 53; of 128 212 / 101; 2,000 tokens 3,820 / 1,100; one token each
-// of 8 sequences of 2,000 keys (a block per token then) 597 / 170; of one key 3.2 / 4.5.
+// Four heads of a KV head at a time (attention_rows_kernel; float32, heads of 64 or 128 that come in fours per KV head): a warp
+// takes four heads of a token, and its block brings 32 keys and values at a time to shared memory by cp.async.  For the
+// scores a lane has a key and forms its four products with the heads; the softmax is that of four runs of eight lanes; for
+// the values a lane has its dimensions.  Every sum is formed in the order of the other kernel, operation by operation, so a
+// row's bits do not depend on which of the two ran.  Bound by instructions (about nine per head and key and 32 lanes) where
+// tokens share their keys, else by the chain of one warp.  us row by row / this, 32 heads on 8: 333 tokens, heads of 64
+// 156 / 53, of 128 212 / 100; one token each of 1, 8 and 48 sequences, heads of 64, on one key 3.0 / 2.6, 3.2 / 2.7, 3.4 / 2.8,
+// on 40 keys 14 / 6, 14 / 6, 14 / 8, on 2,000 keys 587 / 168, 590 / 169, 1,390 / 192; of 200 sequences with heads of 128 on one
+// key 7.5 / 11.6 (the one case that was seen slower), on 16 keys 16 / 14, on 500 keys 936 / 210.
 #include "common.cuh"
 
 #define KEYS 8      // keys that a warp takes at a time; the exchanges below are written for 8
@@ -30,23 +33,13 @@ __device__ __forceinline__ size_t key_place(const int* bt, int s, int K, int kh,
   return (((size_t)bt[s / page_size] * K + kh) * page_size + s % page_size) * D;
 }
 
+// One row, a query head of a token at position pos, by one warp: q and o its D numbers, bt its sequence's row of the block table.
 // WHOLE: pages hold a multiple of KEYS keys, so that a run of them lies in one page; others look up every key
 template <typename T, int DPL, bool WHOLE>
-__global__ void attention_simt_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out,
-                                      const T* __restrict__ k_pages, const T* __restrict__ v_pages,
-                                      const int* __restrict__ block_table, int table_width,
-                                      const int* __restrict__ tok_pos, const int* __restrict__ tok_seq,
-                                      int n_tokens, int H, int K, int D, int page_size, float scale, int window) {
+__device__ __forceinline__ void walk_row(const T* __restrict__ qv, T* __restrict__ o, const T* __restrict__ k_pages,
+                                         const T* __restrict__ v_pages, const int* __restrict__ bt, int pos, int kh, int K, int D,
+                                         int page_size, float scale, int window) {
   const int lane = threadIdx.x & 31;
-  const long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (w >= (long long)n_tokens * H) return;
-  const int t = (int)(w / H), h = (int)(w - (long long)t * H);
-  const int b = tok_seq[t];
-  T* o = out + ((size_t)t * H + h) * D;
-  if (b < 0) return;
-  const int pos = tok_pos[t];
-  const int kh = h / (H / K);
-  const T* qv = q + (size_t)t * q_stride + (size_t)h * D;
   float qr[DPL], acc[DPL];
 #pragma unroll
   for (int j = 0; j < DPL; ++j) {
@@ -56,7 +49,6 @@ __global__ void attention_simt_kernel(const T* __restrict__ q, int q_stride, T* 
   }
   float m = -INFINITY, l = 0.f;
   const int lo = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
-  const int* bt = block_table + (size_t)b * table_width;
   // KEYS keys at a time (a run starts at a multiple of KEYS, so it does not depend on where the walk began)
   for (int s0 = lo - lo % KEYS; s0 <= pos; s0 += KEYS) {
     const size_t base = key_place(bt, s0, K, kh, page_size, D);
@@ -123,41 +115,68 @@ __global__ void attention_simt_kernel(const T* __restrict__ q, int q_stride, T* 
   }
 }
 
+template <typename T, int DPL, bool WHOLE>
+__global__ void attention_simt_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out,
+                                      const T* __restrict__ k_pages, const T* __restrict__ v_pages,
+                                      const int* __restrict__ block_table, int table_width,
+                                      const int* __restrict__ tok_pos, const int* __restrict__ tok_seq,
+                                      int n_tokens, int H, int K, int D, int page_size, float scale, int window) {
+  const long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (w >= (long long)n_tokens * H) return;
+  const int t = (int)(w / H), h = (int)(w - (long long)t * H);
+  const int b = tok_seq[t];
+  if (b < 0) return;
+  walk_row<T, DPL, WHOLE>(q + (size_t)t * q_stride + (size_t)h * D, out + ((size_t)t * H + h) * D, k_pages, v_pages,
+                          block_table + (size_t)b * table_width, tok_pos[t], h / (H / K), K, D, page_size, scale, window);
+}
+
 // float32, D = 32 DPL, pages of a multiple of KEYS keys; see the head of the file.
+// TOKENS of a block: 8, a run of its sequence's, each a warp; or 1, of any sequence, whose four heads are one warp's (other
+// warps help to load).  A token that sees a single run of KEYS keys goes row by row, without shared memory.
 #define ROWS 4             // heads of a warp
-#define ROW_WARPS 8        // tokens of a block
 #define STEP 32            // keys at a time
-template <int DPL> struct RowsShape {
+template <int DPL, int TOKENS, int WARPS, int BUFFERS> struct RowsShape {
   static constexpr int D = 32 * DPL;
   static constexpr int KP = D + 4;                                   // a lane per key reads 16 bytes of its row: no bank twice
   static constexpr int TILE = STEP * (KP + D);                       // floats of a step's keys and values
-  static constexpr int Q = 2 * TILE, P = Q + ROW_WARPS * ROWS * D, SMEM = (P + ROW_WARPS * ROWS * STEP) * 4;
+  static constexpr int Q = BUFFERS * TILE, P = Q + TOKENS * ROWS * D, SMEM = (P + TOKENS * ROWS * STEP) * 4;
 };
 
-template <int DPL>
-__global__ void __launch_bounds__(ROW_WARPS * 32)
+template <int DPL, int TOKENS, int WARPS, int BUFFERS>
+__global__ void __launch_bounds__(WARPS * 32)
 attention_rows_kernel(const float* __restrict__ q, int q_stride, float* __restrict__ out, const float* __restrict__ k_pages,
                       const float* __restrict__ v_pages, const int* __restrict__ block_table, int table_width,
                       const int* __restrict__ tok_pos, const int* __restrict__ tok_seq, const int* __restrict__ cu_q, int n_seqs,
                       int n_tokens, int H, int K, int page_size, float scale, int window) {
-  using S = RowsShape<DPL>;
-  constexpr int D = S::D, T = ROW_WARPS * 32;
+  using S = RowsShape<DPL, TOKENS, WARPS, BUFFERS>;
+  constexpr int D = S::D, T = WARPS * 32;
   extern __shared__ __align__(16) float sm[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int h = blockIdx.y * ROWS, kh = h / (H / K);
-  // this block's tokens: one, or the next of its sequence's runs of ROW_WARPS (the last ones, which see most keys, first)
+  // this block's tokens: one, or the next of its sequence's runs of TOKENS (the last ones, which see most keys, first); a lane
+  // per sequence looks for it
   int t0 = blockIdx.x, t_end = t0 + 1;
-  if (cu_q) {
+  if (TOKENS > 1) {
     int tile = gridDim.x - 1 - blockIdx.x;
     t_end = t0 = 0;
-    for (int i = 0; i < n_seqs; ++i) {
-      const int begin = cu_q[i], end = min(cu_q[i + 1], n_tokens), tiles = (end - begin + ROW_WARPS - 1) / ROW_WARPS;
-      if (tile < tiles) {
-        t0 = begin + tile * ROW_WARPS;
-        t_end = min(end, t0 + ROW_WARPS);
+    for (int i0 = 0; i0 < n_seqs; i0 += 32) {
+      const int i = i0 + lane, begin = i < n_seqs ? cu_q[i] : 0, end = i < n_seqs ? min(cu_q[i + 1], n_tokens) : 0;
+      const int tiles = max(0, (end - begin + TOKENS - 1) / TOKENS);
+      int upto = tiles;                            // runs of the lanes up to this one
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int before = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += before;
+      }
+      const unsigned found = __ballot_sync(0xffffffffu, tile < upto);
+      if (found) {
+        const int at = __ffs(found) - 1;
+        const int from = begin + (tile - (upto - tiles)) * TOKENS;
+        t0 = __shfl_sync(0xffffffffu, from, at);
+        t_end = min(__shfl_sync(0xffffffffu, end, at), t0 + TOKENS);
         break;
       }
-      tile -= max(tiles, 0);
+      tile -= __shfl_sync(0xffffffffu, upto, 31);
     }
   }
   if (t0 >= t_end) return;                         // more blocks than runs
@@ -167,6 +186,17 @@ attention_rows_kernel(const float* __restrict__ q, int q_stride, float* __restri
   const bool mine = t < t_end;
   const int pos = mine ? tok_pos[t] : -1;
   const int lo = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
+  const int* bt = block_table + (size_t)b * table_width;
+  if (TOKENS == 1) {
+    const int p = tok_pos[t0];
+    if (p < KEYS) {
+#pragma unroll 1
+      for (int i = h + warp; i < h + ROWS; i += WARPS)
+        walk_row<float, DPL, true>(q + (size_t)t0 * q_stride + (size_t)i * D, out + ((size_t)t0 * H + i) * D, k_pages, v_pages, bt, p,
+                                   kh, K, D, page_size, scale, window);
+      return;
+    }
+  }
   float* q_s = sm + S::Q + warp * ROWS * D;
   float* p_s = sm + S::P + warp * ROWS * STEP;
   if (mine) {
@@ -189,7 +219,6 @@ attention_rows_kernel(const float* __restrict__ q, int q_stride, float* __restri
     from = min(from, (window > 0 && p - window + 1 > 0) ? p - window + 1 : 0);
   }
   from -= from % KEYS;
-  const int* bt = block_table + (size_t)b * table_width;
   auto stage = [&](int s0, int buf) {
     if (s0 <= to) {
       float* k_t = sm + buf * S::TILE;
@@ -202,11 +231,11 @@ attention_rows_kernel(const float* __restrict__ q, int q_stride, float* __restri
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  stage(from, 0);
   int buf = 0;
-  for (int s0 = from; s0 <= to; s0 += STEP, buf ^= 1) {
-    stage(s0 + STEP, buf ^ 1);
-    asm volatile("cp.async.wait_group 1;" ::: "memory");
+  if (BUFFERS == 2) stage(from, 0);
+  for (int s0 = from; s0 <= to; s0 += STEP, buf ^= BUFFERS - 1) {
+    stage(BUFFERS == 2 ? s0 + STEP : s0, BUFFERS == 2 ? buf ^ 1 : 0);
+    asm volatile("cp.async.wait_group %0;" ::"n"(BUFFERS - 1) : "memory");
     __syncthreads();
     if (mine && s0 <= pos && s0 + STEP > lo) {
       const float *k_row = sm + buf * S::TILE + lane * S::KP, *v_t = sm + buf * S::TILE + STEP * S::KP;
@@ -324,19 +353,42 @@ attention_rows_kernel(const float* __restrict__ q, int q_stride, float* __restri
   }
 }
 
-template <int DPL>
-static int launch_rows(const float* q, int q_stride, float* out, const float* k_pages, const float* v_pages, const int* block_table,
-                       int table_width, const int* tok_pos, const int* tok_seq, const int* cu_q, int n_seqs, int n_tokens, int H,
-                       int K, int page_size, float scale, int window, cudaStream_t stream) {
-  constexpr int smem = RowsShape<DPL>::SMEM;
-  const cudaError_t e = cudaFuncSetAttribute(attention_rows_kernel<DPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+struct RowsArgs {
+  const float* q;
+  int q_stride;
+  float* out;
+  const float *k_pages, *v_pages;
+  const int* block_table;
+  int table_width;
+  const int *tok_pos, *tok_seq, *cu_q;
+  int n_seqs, n_tokens, H, K, page_size;
+  float scale;
+  int window;
+  cudaStream_t stream;
+};
+template <int DPL, int TOKENS, int WARPS, int BUFFERS>
+static int launch_rows(const RowsArgs& a) {
+  using S = RowsShape<DPL, TOKENS, WARPS, BUFFERS>;
+  auto kernel = attention_rows_kernel<DPL, TOKENS, WARPS, BUFFERS>;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM);
   if (e != cudaSuccess) return AB_CUDA_ERR + (int)e;
   // (a sequence's last run may be short: at most n_seqs more than the tokens fill)
-  const dim3 grid((unsigned)(cu_q ? (n_tokens + ROW_WARPS - 1) / ROW_WARPS + n_seqs : n_tokens), (unsigned)(H / ROWS));
-  attention_rows_kernel<DPL><<<grid, ROW_WARPS * 32, smem, stream>>>(q, q_stride, out, k_pages, v_pages, block_table, table_width,
-                                                                      tok_pos, tok_seq, cu_q, n_seqs, n_tokens, H, K, page_size,
-                                                                      scale, window);
+  const dim3 grid((unsigned)(TOKENS > 1 ? (a.n_tokens + TOKENS - 1) / TOKENS + a.n_seqs : a.n_tokens), (unsigned)(a.H / ROWS));
+  kernel<<<grid, WARPS * 32, S::SMEM, a.stream>>>(a.q, a.q_stride, a.out, a.k_pages, a.v_pages, a.block_table, a.table_width,
+                                                     a.tok_pos, a.tok_seq, a.cu_q, a.n_seqs, a.n_tokens, a.H, a.K, a.page_size,
+                                                     a.scale, a.window);
   return ab_launch_status();
+}
+// Runs of eight tokens where sequences bring four or more on average or the runs leave processors idle (32 heads of 128, us in
+// runs / token by token: 100 sequences of 3 tokens on 40 keys 76 / 37, 8 of 3 on 700 87 / 97), else a block per token: while
+// there is a processor for each, with seven warps that help to load (one token on 4,000 keys, 1 / 4 / 8 warps 626 / 533 /
+// 460); up to three blocks a processor, with three (48 tokens of 32 heads on 500 keys 87 / 74 / 181); more, one warp and one
+// buffer, twelve a processor (200 tokens 210 / 282 / 660).
+template <int DPL>
+static int launch_rows(RowsArgs a) {
+  if (a.cu_q && (a.n_tokens >= 4LL * a.n_seqs || (long long)a.n_seqs * (a.H / ROWS) <= 148)) return launch_rows<DPL, 8, 8, 2>(a);
+  const long long blocks = (long long)a.n_tokens * (a.H / ROWS);
+  return blocks <= 148 ? launch_rows<DPL, 1, 8, 2>(a) : blocks <= 444 ? launch_rows<DPL, 1, 4, 2>(a) : launch_rows<DPL, 1, 1, 1>(a);
 }
 
 template <typename T>
@@ -369,9 +421,9 @@ AB_API int ab_attention_simt_rows(const void* q, int q_stride, void* out, int dt
   if (D <= 0 || D > 256 || H <= 0 || K <= 0 || H % K || page_size <= 0) return AB_BAD_ARG;
   if ((cu_q || single) && dtype == AB_F32 && (D == 64 || D == 128) && H / K % ROWS == 0 && H / ROWS <= 65535 && page_size % KEYS == 0 &&
       (((uintptr_t)k_pages | (uintptr_t)v_pages) & 15) == 0) {
-    return (D == 64 ? launch_rows<2> : launch_rows<4>)((const float*)q, q_stride, (float*)out, (const float*)k_pages,
-                                                       (const float*)v_pages, block_table, table_width, tok_pos, tok_seq,
-                                                       single ? nullptr : cu_q, n_seqs, n_tokens, H, K, page_size, scale, window, stream);
+    const RowsArgs a{(const float*)q, q_stride, (float*)out, (const float*)k_pages, (const float*)v_pages, block_table, table_width,
+                     tok_pos, tok_seq, single ? nullptr : cu_q, n_seqs, n_tokens, H, K, page_size, scale, window, stream};
+    return D == 64 ? launch_rows<2>(a) : launch_rows<4>(a);
   }
   if (dtype == AB_F32)
     return launch<float>(q, q_stride, out, k_pages, v_pages, block_table, table_width, tok_pos, tok_seq,

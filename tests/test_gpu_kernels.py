@@ -900,3 +900,28 @@ def test_attention_32bit_of_scores_of_minus_infinity(dtype, H, K, D, window):
         assert want.isnan().any() == (b < 2) and not want.isnan().all()
         close(outs[0][t0:t0 + n].view(n, H, D), want.nan_to_num(9.0), dtype, f"sequence {b}")
         t0 += n
+
+
+@pytest.mark.parametrize("H,K,D", [(16, 4, 64), (16, 2, 128)])
+@pytest.mark.parametrize("n,tokens,longest", [(9, 1, 100), (24, 1, 100), (48, 1, 100), (130, 1, 100), (150, 1, 9), (70, 2, 90),
+                                              (70, 9, 60), (33, 4, 200), (12, 3, 200)])
+def test_attention_32bit_forms_have_the_same_bits(H, K, D, n, tokens, longest):
+    """Up to 148 blocks of one token, up to 444 and more; sequences of few tokens token by token or in runs, more of them than a
+    warp has lanes; sequences of up to eight keys among the others: all as row by row."""
+    from alpacca_b200 import ops
+    lengths = [max(tokens, 1 + (longest * (7 * b + 3)) % (longest + 1)) for b in range(n)]
+    q_lens = [max(1, tokens - b % 3) for b in range(n)]
+    table, kp, vp = make_paged(lengths, sum(-(-x // 64) for x in lengths), K, D, torch.float32, seed=1)
+    kp.copy_(rnd(*kp.shape, seed=2))
+    vp.copy_(rnd(*vp.shape, seed=3))
+    T = sum(q_lens)
+    qkv = rnd(T, (H + 2 * K) * D, seed=4)
+    pos = torch.cat([torch.arange(x - q, x) for x, q in zip(lengths, q_lens)]).to(torch.int32).cuda()
+    seq = torch.repeat_interleave(torch.arange(n), torch.tensor(q_lens)).to(torch.int32).cuda()
+    cu = torch.tensor([0] + torch.tensor(q_lens).cumsum(0).tolist(), dtype=torch.int32).cuda()
+    outs = []
+    for form in [{}, {"cu_q": cu}] + ([{"single": True}] if tokens == 1 else []):
+        out = torch.full((T, H * D), 7.0, device="cuda")
+        ops.attention_simt(qkv, out, kp, vp, table, pos, seq, T, H, K, D, D ** -0.5, 20 if longest == 60 else 0, **form)
+        outs.append(out)
+    assert all(torch.equal(o, outs[0]) for o in outs) and not (outs[0] == 7.0).any()
