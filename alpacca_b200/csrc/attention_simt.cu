@@ -413,10 +413,10 @@ static int launch(const void* q, int q_stride, void* out, const void* k_pages, c
 
 // cu_q (int [n_seqs + 1], or null): where the sequences' tokens begin, in prompts.  `single`: one token per sequence.  With one of
 // the two, the kernel of four heads is taken where it can be; the results are the same.
-AB_API int ab_attention_simt_rows(const void* q, int q_stride, void* out, int dtype, const void* k_pages,
-                                  const void* v_pages, const int* block_table, int table_width, const int* tok_pos,
-                                  const int* tok_seq, const int* cu_q, int n_seqs, int single, int n_tokens, int H, int K, int D,
-                                  int page_size, float scale, int window, cudaStream_t stream) {
+AB_API int ab_attention_simt(const void* q, int q_stride, void* out, int dtype, const void* k_pages, const void* v_pages,
+                             const int* block_table, int table_width, const int* tok_pos, const int* tok_seq, const int* cu_q,
+                             int n_seqs, int single, int n_tokens, int H, int K, int D, int page_size, float scale, int window,
+                             cudaStream_t stream) {
   if (n_tokens <= 0) return AB_OK;
   if (D <= 0 || D > 256 || H <= 0 || K <= 0 || H % K || page_size <= 0) return AB_BAD_ARG;
   if ((cu_q || single) && dtype == AB_F32 && (D == 64 || D == 128) && H / K % ROWS == 0 && H / ROWS <= 65535 && page_size % KEYS == 0 &&
@@ -432,12 +432,4 @@ AB_API int ab_attention_simt_rows(const void* q, int q_stride, void* out, int dt
     return launch<bf16>(q, q_stride, out, k_pages, v_pages, block_table, table_width, tok_pos, tok_seq,
                         n_tokens, H, K, D, page_size, scale, window, stream);
   return AB_BAD_ARG;
-}
-
-AB_API int ab_attention_simt(const void* q, int q_stride, void* out, int dtype, const void* k_pages,
-                             const void* v_pages, const int* block_table, int table_width, const int* tok_pos,
-                             const int* tok_seq, int n_tokens, int H, int K, int D, int page_size, float scale,
-                             int window, cudaStream_t stream) {
-  return ab_attention_simt_rows(q, q_stride, out, dtype, k_pages, v_pages, block_table, table_width, tok_pos, tok_seq, nullptr, 0,
-                                0, n_tokens, H, K, D, page_size, scale, window, stream);
 }

@@ -296,7 +296,7 @@ def attention_simt(qkv, out, k_pages, v_pages, block_table, tok_pos, tok_seq, n_
     page_size = k_pages.shape[2]
     _need(tuple(k_pages.shape[1:]) == (K, page_size, D) and k_pages.shape == v_pages.shape
           and k_pages.is_contiguous() and v_pages.is_contiguous(), "attention: cache pages [n_pages,K,page,D]")
-    _check(_lib("attention_simt").ab_attention_simt_rows(
+    _check(_lib("attention_simt").ab_attention_simt(
         _p(qkv), qkv.shape[-1], _p(out), _dt(qkv), _p(k_pages), _p(v_pages), _p(block_table),
         block_table.shape[1], _p(tok_pos), _p(tok_seq), _p(cu_q), n_seqs, 1 if single else 0, n_tokens, H, K, D, page_size,
         ctypes.c_float(scale), int(window or 0), _stream()), "attention_simt")
