@@ -679,16 +679,18 @@ def test_gemm_f32_ragged_k(M, N, K):
     assert ((out[:M].double() - want).abs() <= bound).all() and (out[M] == 7.0).all()
 
 
-@pytest.mark.parametrize("M,K", [(1, 96), (16, 2048), (40, 1100), (130, 513)])
-def test_gemm_f32_extreme_numbers(M, K):
-    """Numbers that no bfloat16 holds (above its largest), infinities and NaNs go where plain multiply-adds take them; numbers of
-    very unlike sizes, and of one sign, keep the bound of the tiles' test."""
+@pytest.mark.parametrize("M,K,largest", [(1, 96, True), (1, 96, False), (1, 2048, False), (16, 2048, True), (16, 2048, False),
+                                         (40, 1100, True), (130, 513, True), (130, 513, False)])
+def test_gemm_f32_extreme_numbers(M, K, largest):
+    """Numbers that no bfloat16 holds (above its largest; with `largest`, in the first row), infinities and NaNs go where plain
+    multiply-adds take them; numbers of very unlike sizes, and of one sign, keep the bound of the tiles' test."""
     from alpacca_b200 import ops
     N = 150
     a, w = rnd(M, K, seed=1), rnd(N, K, seed=2).abs()
     a *= torch.exp2(torch.randint(-30, 30, (M, K), generator=torch.Generator().manual_seed(3)).float()).cuda()
     a[:, 5], w[3, 7], w[4, 7] = 1.0, float("inf"), float("nan")
-    a[0, 9], w[:, 9] = 3.4e38, 1e-3
+    if largest:
+        a[0, 9], w[:, 9] = 3.4e38, 1e-3
     if M > 1:
         a[M // 2, 11] = float("-inf")
     out = torch.empty(M, N, device="cuda")
@@ -925,3 +927,28 @@ def test_attention_32bit_forms_have_the_same_bits(H, K, D, n, tokens, longest):
         ops.attention_simt(qkv, out, kp, vp, table, pos, seq, T, H, K, D, D ** -0.5, 20 if longest == 60 else 0, **form)
         outs.append(out)
     assert all(torch.equal(o, outs[0]) for o in outs) and not (outs[0] == 7.0).any()
+
+
+@pytest.mark.parametrize("M,rows_per_tile", [(1, 16), (20, 32), (64, 64), (96, 96)])
+@pytest.mark.parametrize("K,runs", [(1000, 8), (700, 6), (420, 4), (300, 3)])
+def test_gemm_f32_bits_do_not_depend_on_how_runs_are_shared(M, rows_per_tile, K, runs):
+    """All runs of a tile in one CTA (many tiles), where the sums of the runs before wait in tensor memory, against a run per CTA
+    (few tiles): the same bits, and right.  Bound: that of the tiles' test."""
+    import ctypes
+    from alpacca_b200 import ops
+    N, narrow = 32 * 4008, slice(17 * 128, 17 * 128 + 150)
+    plans = []
+    for cols in (N, 150):
+        plan = (ctypes.c_int * 4)()
+        ops._lib("gemm_f32").ab_gemm_f32_plan(M, cols, K, plan)
+        plans.append(tuple(plan))
+    assert plans[0][1:] == (rows_per_tile, 8, 1) and plans[1][1:] == (rows_per_tile, 1, runs), plans
+    a, w = rnd(M, K, seed=1), rnd(4008, K, seed=2)
+    wide, out = torch.empty(M, N, device="cuda"), torch.empty(M, 150, device="cuda")
+    ops.gemm_f32(a, w.repeat(32, 1), wide)
+    ops.gemm_f32(a, w[narrow].contiguous(), out)
+    assert torch.equal(wide[:, narrow], out) and torch.equal(wide.view(M, 32, 4008), wide[:, None, :4008].expand(M, 32, 4008))
+    wide = wide[:, :4008]
+    bound = 2.0 ** -22 * a.double().norm(dim=1)[:, None] * w.double().norm(dim=1)[None]
+    assert ((wide.double() - a.double() @ w.double().T).abs() <= bound).all()
+    assert ops.gemm_f32_status() == 0
