@@ -2,19 +2,21 @@
 //
 // Every 32-bit number is split into three bfloat16 numbers that add up to it exactly (x = h + m + l: h is x rounded,
 // m the rest rounded, l what is then left, at most eight bits).  A product needs six of the nine partial products,
-//   a w = ah wh + (ah wm + am wh) + (ah wl + am wm + al wh)        the other three are below 2^-26 of |a w|,
-// each exact in 32 bits, summed by tcgen05.mma in three 32-bit accumulators in tensor memory, one per bracket.  The sums
+//   a w = ah wh + (ah wm + am wh) + (ah wl + am wm + al wh)
+// each exact in 32 bits.  (|m| is up to 2^-8 |x|, |l| up to 2^-17 |x|, so the other three are up to about 2^-24 of |a w|, of
+// either sign.)  They are summed by tcgen05.mma in three 32-bit accumulators in tensor memory, one per bracket.  The sums
 // of the tensor cores cut off instead of rounding, so the leading accumulator holds 32 k only: adding warps then add it to
 // a rounded 32-bit sum in registers.  The two others are 2^-8 smaller and run to the end of a run of k.
 // Error against 64 bits, root mean square over |a| |w| (before: multiply-adds in 32 bits): normal numbers 2.0e-9 at 2,048 k
-// (4.7e-9), 1.4e-9 at 8,192 (4.5e-9), 5.6e-9 at 128 (1.3e-8); all of one sign 4.2e-8 at 2,048 (4.7e-8).  A layer of the 1B
-// shape 2.5e-7 (5.4e-7).
+// (4.7e-9), 1.4e-9 at 8,192 (4.5e-9), 5.5e-9 at 128 (1.3e-8), 7.4e-9 at 48 (1.4e-8); all of one sign 3.8e-8 at 2,048
+// (4.3e-8), 3.5e-8 at 48 (3.9e-8).  A layer of the 1B shape 2.5e-7 (5.4e-7).  Below 48 k the roundings weigh more than those
+// of multiply-adds, which are taken there (`gemm_f32_short_kernel`).
 //
 // The order of an output's sum depends on K alone: the k range is cut into up to GROUPS runs (of a multiple of BK, at
-// least SHORTEST), a run into stages of 32; the first four runs are added in ascending order, the others too, then both.  So a value does not depend on M, on
-// the tile it falls into, on whether the runs of a tile are computed by one CTA or by a cluster of CTAs, or on what other
-// rows are in the batch: the same token gives the same bits alone and in any batch.  This is the matrix product of the
-// 32-bit path (the reference's float32 path uses BLAS SGEMM, alpacca/tensor.py:91-97).
+// least SHORTEST), a run into stages of 32; the first four runs are added in ascending order, the others too, then both.
+// So a value does not depend on M, on the tile it falls into, on whether the runs of a tile are computed by one CTA or by
+// a cluster of CTAs, or on what other rows are in the batch: the same token gives the same bits alone and in any batch.
+// This is the matrix product of the 32-bit path (the reference's float32 path uses BLAS SGEMM, alpacca/tensor.py:91-97).
 //
 // The parts are those of 2^16 times a number, so that the smallest number's last bit is one of a bfloat16 too, and outputs
 // are multiplied by 2^-32: powers of two, which change no other bit.  A number of 2^112 or more splits into infinities and
@@ -25,13 +27,16 @@
 // by cp.async into a ring in shared memory (each thread only what it splits itself, so nobody waits for anybody), split
 // them and store the parts in the swizzled form that the MMA reads; adding warps move the leading accumulator; one lane of
 // another warp issues the MMAs, four per 16 k: [wm|wl] and [wh|wm] lie side by side, so that two MMAs do the work of four.
-// What bounds it: for many rows the splitting and adding instructions (some 1,400 clocks a stage at n = 128, the tensor cores
-// 768); for few rows the latency of a stage, hidden by two CTAs per processor, and HBM.
-// us before (multiply-adds) / now: 333 rows of q|k|v, o, gate|up and down of the 1B shape 123 / 44, 87 / 44, 570 / 261,
-// 316 / 154; 64 rows 34 / 25, 24 / 24, 114 / 61, 81 / 62; 17 rows 22 / 17, 15 / 15, 67 / 52, 50 / 45; one row 11.6 / 12.2,
-// 10.8 / 11.1, 35.8 / 33.6, 35.5 / 31.7.  2,048 rows of 16384x2048: 2,960 / 1,242 (111 TFLOP/s, 46 before).
-// Tried: 16 warps that split and add in turn (333 rows of gate|up 243, one row of q|k|v 15.8); rounding in integers in place of the
-// conversion instruction (the same); two leading accumulators (one row 0.8 us slower a product).
+// What bounds it: for many rows the splitting and adding instructions (some 1,400 clocks a stage at n = 128, the tensor
+// cores 768); for few rows the latency of a stage, hidden by two CTAs per processor, and HBM.
+// us multiply-adds on the FMA pipes (before) / this: 333 rows of q|k|v, o, gate|up and down of the 1B shape 123 / 45, 87 / 45,
+// 571 / 266, 315 / 145; 64 rows 34 / 25, 24 / 24, 114 / 63, 81 / 61; 17 rows 22 / 16, 15 / 15, 67 / 49, 50 / 43; one row
+// 11.6 / 12.3, 11.0 / 11.2, 35.9 / 33.6, 35.5 / 30.5.  2,048 rows of 16384x2048: 2,960 / 1,314 (105 TFLOP/s, 46 before).
+// Its chain of steps (copy, split, multiply, add, store) is longer than that of multiply-adds: few rows of small matrices
+// take 0.5 to 1.8 us more (one row of 2048x128 3.8 / 5.6, of 512x1024 4.7 / 6.2; 333 rows of 2048x128 11.9 / 8.4).
+// Tried: 16 warps that split and add in turn (333 rows of gate|up 243, one row of q|k|v 15.8); rounding in integers in place
+// of the conversion instruction (the same); two leading accumulators (one row 0.8 us slower a product), four of them where a
+// CTA has four stages (one row of 2048x128 0.2 us faster, 333 rows of 16384x128 1 us slower).
 //
 // Every wait on an mbarrier is bounded; a thread that gives up leaves a code in `gemm_f32_stuck`, all roles fall through
 // to the end, where TMEM is given back, and the outputs are NaN until `plain_rows` has formed them.
@@ -232,8 +237,8 @@ template <int NT> struct F32Shape {
   static_assert(CTAS * (SMEM + 1024) <= 233472, "what a CTA may have");
 };
 
-// PER: the runs of a CTA: all of them, half of GROUPS or one.  `cs` CTAs then share a tile as a cluster, and each adds up its
-// part of the tile through distributed shared memory.  VEC: both operands' rows can be copied 16 bytes at a time.
+// PER: the runs of a CTA: all of them, half of GROUPS or one.  `cs` CTAs then share a tile as a cluster, and each adds up
+// its part of the tile through distributed shared memory.  VEC: both operands' rows can be copied 16 bytes at a time.
 template <int NT, bool VEC, int PER>
 __global__ void __launch_bounds__(F32Shape<NT>::THREADS, F32Shape<NT>::CTAS)
 gemm_f32_nt_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw,

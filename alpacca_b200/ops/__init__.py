@@ -305,7 +305,8 @@ def attention_simt(qkv, out, k_pages, v_pages, block_table, tok_pos, tok_seq, n_
 
 def gemm_f32(a, w, out, bias=None, n_rows=None):
     """out[M,N] = a[M,K] @ w[N,K]^T (+ bias) with the precision of float32 sums in a fixed order: operands as exact sums of
-    three bfloat16 parts on the tensor cores."""
+    three bfloat16 parts on the tensor cores (numbers of every size; what is not finite, and fewer than 48 k, by
+    multiply-adds)."""
     _cuda(a, w, out, bias)
     _need(a.dtype == torch.float32 and w.dtype == torch.float32 and out.dtype == torch.float32,
           "gemm_f32 takes float32 tensors")

@@ -2,7 +2,9 @@
 
 Several checkpoint matrices that read the same input can be held as one fused
 matrix (q|k|v, gate|up).  In the 32-bit path the product is the package's own
-FMA kernel; in the bfloat16 path it is the skinny-matrix kernel for the few rows
+kernel with the precision of 32-bit sums (csrc/gemm_f32.cu: operands split exactly
+into bfloat16 parts on the tensor cores, multiply-adds for few k); in the bfloat16
+path it is the skinny-matrix kernel for the few rows
 of a decode step and the library matrix product otherwise (the reference uses
 BLAS for every product: alpacca/tensor.py:82-97).
 """
