@@ -772,8 +772,10 @@ def attention(qkv, out, cache, ctx, H, K, D, scale, window=0):
     # Steps that are known to reach no further than one run of eight keys go row by row (us row by row / four heads: one prompt
     # of 8 tokens, 32 heads of 128, 5.0 / 7.0; 100 of 5 tokens 14 / 35); a captured step's replays may reach further
     short = (getattr(ctx, "max_kv_len", None) or 9) <= 8 and not torch.cuda.is_current_stream_capturing()
-    single = ctx.is_decode and not short
-    cu_q = None if ctx.is_decode or short else ctx.cu_q[:ctx.n_seqs + 1]
+    single = getattr(ctx, "is_decode", False) and not short
+    cu_q = None if single or short else getattr(ctx, "cu_q", None)
+    if cu_q is not None:
+        cu_q = cu_q[:ctx.n_seqs + 1]
     return attention_simt(qkv, out, cache.k, cache.v, cache.block_table, ctx.tok_pos, ctx.tok_seq,
                           ctx.n_tokens, H, K, D, scale, window, cu_q=cu_q, single=single)
 

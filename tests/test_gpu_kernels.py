@@ -952,3 +952,28 @@ def test_gemm_f32_bits_do_not_depend_on_how_runs_are_shared(M, rows_per_tile, K,
     bound = 2.0 ** -22 * a.double().norm(dim=1)[:, None] * w.double().norm(dim=1)[None]
     assert ((wide.double() - a.double() @ w.double().T).abs() <= bound).all()
     assert ops.gemm_f32_status() == 0
+
+
+@pytest.mark.parametrize("n", [3, 40])
+def test_attention_32bit_of_a_step_that_only_names_its_tokens(n):
+    """The 32-bit attention needs of a step its tokens' sequences and positions, not where the sequences begin; steps of up to
+    eight keys and longer ones give the bits of the same step with everything named."""
+    from alpacca_b200 import ops
+    from alpacca_b200.cache import KVLayerView
+    from types import SimpleNamespace
+    H, K, D = 8, 2, 64
+    table, kp, vp = make_paged([n], 2, K, D, torch.float32, seed=1)
+    kp.copy_(rnd(*kp.shape, seed=2))
+    vp.copy_(rnd(*vp.shape, seed=3))
+    qkv = rnd(n, (H + 2 * K) * D, seed=4)
+    pos, seq = torch.arange(n, dtype=torch.int32).cuda(), torch.zeros(n, dtype=torch.int32).cuda()
+    named = dict(is_decode=False, n_seqs=1, cu_q=torch.tensor([0, n], dtype=torch.int32).cuda(), max_kv_len=n)
+    outs = []
+    for more in ({}, named):
+        ctx = SimpleNamespace(tok_pos=pos, tok_seq=seq, n_tokens=n, **more)
+        outs.append(torch.empty(n, H * D, device="cuda"))
+        ops.attention(qkv, outs[-1], KVLayerView(kp, vp, table, None), ctx, H, K, D, D ** -0.5)
+    assert torch.equal(outs[0], outs[1])
+    want = ref_attention(qkv.double().cpu().view(n, -1, D)[:, :H], *(p[table[0].long()].transpose(1, 2).reshape(-1, K, D)[:n].double().cpu()
+                                                                     for p in (kp, vp)), pos.cpu(), D ** -0.5)
+    close(outs[0].view(n, H, D), want, "float32")
