@@ -22,9 +22,9 @@
 // the values a lane has its dimensions.  Every sum is formed in the order of the other kernel, operation by operation, so a
 // row's bits do not depend on which of the two ran.  Bound by instructions (about nine per head and key and 32 lanes) where
 // tokens share their keys, else by the chain of one warp.  us row by row / this, 32 heads on 8: 333 tokens, heads of 64
-// 156 / 53, of 128 212 / 100; one token each of 1, 8 and 48 sequences, heads of 64, on one key 3.0 / 2.6, 3.2 / 2.7, 3.4 / 2.8,
-// on 40 keys 14 / 6, 14 / 6, 14 / 8, on 2,000 keys 587 / 168, 590 / 169, 1,390 / 192; of 200 sequences with heads of 128 on one
-// key 7.5 / 11.6 (the one case that was seen slower), on 16 keys 16 / 14, on 500 keys 936 / 210.
+// 156 / 53, of 128 212 / 101; one token each of 1, 8 and 48 sequences, heads of 64, on one key 3.1 / 2.7, 3.2 / 2.8, 3.5 / 3.0,
+// on 16 keys 6.7 / 4.5, 6.9 / 4.6, 7.3 / 5.0; of 8 on 2,000 keys 589 / 169, of 48 on 500 keys 271 / 51; of 200 sequences with
+// heads of 128 on one key 7.5 / 11.6 (the one case that was seen slower), on 40 keys 39 / 26, on 500 keys 914 / 211.
 #include "common.cuh"
 
 #define KEYS 8      // keys that a warp takes at a time; the exchanges below are written for 8
